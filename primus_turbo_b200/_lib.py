@@ -120,14 +120,15 @@ _GEMM_ENTRY_POINTS = ("ptb_gemm_fp8", "ptb_gemm_mxfp8", "ptb_grouped_gemm_fp8", 
                       "ptb_grouped_gemm_mxfp8", "ptb_grouped_gemm_mxfp8_variable_k")
 # PTB_NVTX=1: one NVTX range per C-ABI call, named after the entry point (timeline tools show them)
 _NVTX = os.environ.get("PTB_NVTX", "0") not in ("", "0")
-launch_count = 0  # running total of kernels this process enqueued through the C ABI
+_launches = 0  # kernels enqueued by ``call``
+_native_launches = lambda: 0  # noqa: E731  (kernels enqueued by the native host path, once that is loaded)
 _event_log = None  # when a dict: name -> [(start_event, stop_event), ...] on the launching stream
 
 
 def call(name: str, *args) -> None:
     """Invoke one C-ABI entry point: count its launches, optionally bracket it with CUDA events on
     the current stream (see record_kernel_times), raise PtbError on a non-zero status."""
-    global launch_count
+    global _launches
     fn = getattr(lib, name)
     if _NVTX:
         torch.cuda.nvtx.range_push(name)
@@ -136,7 +137,7 @@ def call(name: str, *args) -> None:
         finally:
             torch.cuda.nvtx.range_pop()
         check(rc, name)
-        launch_count += KERNELS_PER_CALL.get(name, 1)
+        _launches += KERNELS_PER_CALL.get(name, 1)
         return
     if _event_log is not None:
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -147,13 +148,19 @@ def call(name: str, *args) -> None:
     else:
         rc = fn(*args)
     check(rc, name)
-    launch_count += KERNELS_PER_CALL.get(name, 1)
+    _launches += KERNELS_PER_CALL.get(name, 1)
     if _DEBUG_STATUS and name in _GEMM_ENTRY_POINTS and not torch.cuda.is_current_stream_capturing():
         # (a stream that is being captured into a graph cannot be waited for: the check is skipped there)
         torch.cuda.synchronize()
         code = gemm_status(reset=True)
         if code != 0:
             raise PtbError(f"{name}: a device-side wait ran out (status {code}); the output is incomplete")
+
+
+def __getattr__(name: str):
+    if name == "launch_count":  # running total of kernels this process enqueued through the C ABI
+        return _launches + _native_launches()
+    raise AttributeError(name)
 
 
 class timed_region:

@@ -20,6 +20,7 @@ from typing import Optional, Union
 
 import torch
 
+from primus_turbo_b200 import _native
 from primus_turbo_b200.pytorch.core.low_precision import (
     Float8QuantConfig,
     Format,
@@ -227,7 +228,31 @@ class FP8GemmMXFunction(torch.autograd.Function):
         return grad_a, grad_b, None, None, None, None, None, None
 
 
-@torch._dynamo.disable(recursive=True, reason="builds QuantizedTensor wrappers inside autograd.Function.forward")
+_TILES = ScalingRecipe(use_2d_block=True)  # how BLOCKWISE and MX weights are quantised
+
+
+def _native_gemm(a, b, trans_a, trans_b, out_dtype, config):
+    """The whole call through the native host path; ``None`` where it has to run in Python."""
+    g = config.granularity
+    if g == ScalingGranularity.BLOCKWISE and config.block_size != 128:
+        return None
+    b_scale = None
+    if isinstance(b, QuantizedTensor):
+        # a weight quantised ahead of time, in inference: its payload in the forward direction is all that is read
+        ok = b.granularity == g and b.block_size == config.block_size and not b._is_grouped_tensor
+        if g in (ScalingGranularity.BLOCKWISE, ScalingGranularity.MX_BLOCKWISE):
+            ok = ok and b.scaling_recipe == _TILES
+        if g in (ScalingGranularity.ROWWISE, ScalingGranularity.MX_BLOCKWISE):
+            ok = ok and b.quantized_axis == (1 if trans_b else 0)
+        if not ok or b.requires_grad or (a.requires_grad and torch.is_grad_enabled()):
+            return None
+        b, b_scale = b.qdata, b.scale_inv
+    elif not _native.usable(b):
+        return None
+    return _native.ext.gemm_fp8(a, b, b_scale, trans_a, trans_b, out_dtype, g.value, _get_fp8_dtype(config.format, True),
+                                _get_fp8_dtype(config.format, False))
+
+
 def gemm_fp8(
     a: Union[torch.Tensor, QuantizedTensor, QuantizedTensorPair],
     b: Union[torch.Tensor, QuantizedTensor, QuantizedTensorPair],
@@ -249,7 +274,16 @@ def gemm_fp8(
     assert b_data.ndim == 2, "Only 2D tensors are supported"
     if out_dtype is None:
         out_dtype = torch.promote_types(a_data.dtype, b_data.dtype)
-    args = (a_data, b_data, a_data_t, b_data_t, trans_a, trans_b, out_dtype, config)
+    if _native.usable(a_data):
+        out = _native_gemm(a_data, b_data, trans_a, trans_b, out_dtype, config)
+        if out is not None:
+            return out
+    return _gemm_fp8_python(a_data, b_data, a_data_t, b_data_t, trans_a, trans_b, out_dtype, config)
+
+
+@torch._dynamo.disable(recursive=True, reason="builds QuantizedTensor wrappers inside autograd.Function.forward")
+def _gemm_fp8_python(*args):
+    config = args[-1]
     if config.granularity == ScalingGranularity.TENSORWISE:
         return FP8GemmTensorFunction.apply(*args)
     if config.granularity == ScalingGranularity.ROWWISE:

@@ -14,6 +14,7 @@ from typing import Optional, Union
 
 import torch
 
+from primus_turbo_b200 import _native
 from primus_turbo_b200.pytorch.core.low_precision import (
     Float8QuantConfig,
     Format,
@@ -301,6 +302,29 @@ class FP8GroupedGemmMXFunc(torch.autograd.Function):
         return grad_a, grad_b, None, None, None, None, None, None, None, None
 
 
+def _native_grouped(a, b, group_lens, group_offs, trans_b, out_dtype, config, num_cu):
+    """The whole call through the native host path; ``None`` where it has to run in Python."""
+    g = config.granularity
+    if g == ScalingGranularity.BLOCKWISE and config.block_size != 128:
+        return None
+    b_scale = None
+    fwd = _get_fp8_dtype(config.format, True)
+    if isinstance(b, QuantizedTensor):
+        # a weight quantised ahead of time, in inference: its payload in the forward direction is all that is read
+        ok = b.granularity == g and b.block_size == config.block_size and not b._is_grouped_tensor
+        if g in (ScalingGranularity.BLOCKWISE, ScalingGranularity.MX_BLOCKWISE):
+            ok = ok and b.scaling_recipe == _WEIGHT_RECIPE and b.real_dtype == fwd
+        if g in (ScalingGranularity.ROWWISE, ScalingGranularity.MX_BLOCKWISE):
+            ok = ok and b.quantized_axis == (2 if trans_b else 1)
+        if not ok or b.requires_grad or (a.requires_grad and torch.is_grad_enabled()):
+            return None
+        b, b_scale = b.qdata, b.scale_inv
+    elif not _native.usable(b):
+        return None
+    return _native.ext.grouped_gemm_fp8(a, b, b_scale, group_lens, group_offs, trans_b, out_dtype, g.value, fwd,
+                                        _get_fp8_dtype(config.format, False), num_cu or 0)
+
+
 def grouped_gemm_fp8(
     a: Union[torch.Tensor, QuantizedTensor, QuantizedTensorPair],
     b: Union[torch.Tensor, QuantizedTensor, QuantizedTensorPair],
@@ -319,12 +343,16 @@ def grouped_gemm_fp8(
     """
     if config is None:
         config = Float8QuantConfig()
-    if group_offs is None:
-        group_offs = group_offs_from_lens(group_lens)
     a_data, a_data_t = (a.data, a.data_t) if isinstance(a, QuantizedTensorPair) else (a, None)
     b_data, b_data_t = (b.data, b.data_t) if isinstance(b, QuantizedTensorPair) else (b, None)
     if out_dtype is None:
         out_dtype = torch.promote_types(a_data.dtype, b_data.dtype)
+    if _native.usable(a_data):
+        out = _native_grouped(a_data, b_data, group_lens, group_offs, trans_b, out_dtype, config, num_cu)
+        if out is not None:
+            return out
+    if group_offs is None:
+        group_offs = group_offs_from_lens(group_lens)
     if config.granularity == ScalingGranularity.TENSORWISE:
         return FP8GroupedGemmTensorFunc.apply(
             a_data, b_data, a_data_t, b_data_t, group_lens, group_offs, trans_b, out_dtype, config, num_cu

@@ -6,6 +6,7 @@ from typing import Optional, Tuple
 
 import torch
 
+from primus_turbo_b200 import _native
 from primus_turbo_b200.pytorch.core.low_precision import ScalingGranularity, ScalingRecipe
 from primus_turbo_b200.pytorch.core.low_precision import MXFP8_BLOCK_SIZE
 from primus_turbo_b200.pytorch.kernels import custom_ops as _ops
@@ -26,6 +27,9 @@ __all__ = [
 ]
 
 
+_BLOCK_OF = {ScalingGranularity.BLOCKWISE: 128, ScalingGranularity.MX_BLOCKWISE: MXFP8_BLOCK_SIZE}
+
+
 def quantize_fp8(
     x: torch.Tensor,
     out_dtype: torch.dtype,
@@ -41,6 +45,19 @@ def quantize_fp8(
     BLOCKWISE: ``block_size`` (128) required; ``scaling_recipe.use_2d_block`` selects one scale per
     128x128 tile (weights), otherwise ``axis`` picks 1x128 (axis 1/-1) or 128x1 (axis 0/-2) blocks.
     """
+    if _native.usable(x) and block_size == _BLOCK_OF.get(granularity, block_size):
+        tiles = scaling_recipe is not None and scaling_recipe.use_2d_block
+        if granularity == ScalingGranularity.MX_BLOCKWISE:
+            _reject_shuffle(scaling_recipe)
+        if granularity == ScalingGranularity.TENSORWISE:
+            along = 0
+        elif axis is None:
+            along = 0 if tiles and granularity == ScalingGranularity.BLOCKWISE else None
+        else:
+            along = axis if axis >= 0 else axis + x.dim()
+        out = None if along is None else _native.ext.quantize(x, out_dtype, granularity.value, along, tiles)
+        if out is not None:
+            return out
     if granularity == ScalingGranularity.TENSORWISE:
         return _ops.quantize_fp8_tensorwise(x, out_dtype)
     if granularity == ScalingGranularity.ROWWISE:
@@ -81,6 +98,16 @@ def quantize_fp8_with_trans(
     scaling_recipe_for_trans: Optional[ScalingRecipe] = None,
 ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
     """One read of x -> (row copy, row scales [M, N/128], column copy [M,N], column scales [M/128, N])."""
+    if _native.usable(x) and granularity in _BLOCK_OF and block_size == _BLOCK_OF[granularity]:
+        if granularity == ScalingGranularity.MX_BLOCKWISE:
+            _reject_shuffle(scaling_recipe)
+            _reject_shuffle(scaling_recipe_for_trans)
+        out = _native.ext.quantize_dual(
+            x, out_dtype, granularity.value, bool(scaling_recipe is not None and scaling_recipe.use_2d_block),
+            bool(scaling_recipe_for_trans is not None and scaling_recipe_for_trans.use_2d_block),
+        )
+        if out is not None:
+            return out
     if granularity == ScalingGranularity.BLOCKWISE:
         assert block_size is not None, "block_size must be specified for BLOCKWISE quantization"
         return _ops.quant_fp8_blockwise_dual(x, out_dtype, block_size)
@@ -181,6 +208,15 @@ def dequantize_fp8(
     scale_inv: torch.Tensor,
     scaling_recipe: Optional[ScalingRecipe] = None,
 ) -> torch.Tensor:
+    if _native.usable(x) and block_size == _BLOCK_OF.get(granularity, block_size):
+        tiles = granularity == ScalingGranularity.BLOCKWISE and scaling_recipe is not None and scaling_recipe.use_2d_block
+        if granularity == ScalingGranularity.TENSORWISE or (axis is None and tiles):
+            along = 0
+        else:
+            along = None if axis is None else axis if axis >= 0 else axis + x.dim()
+        out = None if along is None else _native.ext.dequantize(x, scale_inv, out_dtype, granularity.value, along, tiles)
+        if out is not None:
+            return out
     if granularity == ScalingGranularity.TENSORWISE:
         return _ops.dequantize_fp8(x, scale_inv, out_dtype, 1, 0, 0)
     if granularity == ScalingGranularity.ROWWISE:
