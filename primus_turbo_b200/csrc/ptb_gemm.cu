@@ -1,10 +1,13 @@
 // FP8 GEMM / grouped GEMM for sm_100a: TMA-fed shared-memory ring, tcgen05.mma with the
 // accumulator in tensor memory, per-128-K-block scale promotion in registers, bf16/fp16 epilogue.
 //
+// Two forms of one kernel (CTAS): a 128 x 256 tile per CTA, or a 256 x 256 tile per pair of CTAs on neighbouring SMs
+// (tcgen05 cta_group::2: each CTA loads its own 128 rows of A and half of B, and holds its own 128 output rows).
+//
 // One persistent CTA per SM, 384 threads:
-//   warp 0      TMA producer (one lane): fills a 3-stage (4 without output staging) ring of {A 128x128, B 256x128} FP8 tiles,
+//   warp 0      TMA producer (one lane): fills a ring of {A 128x128, B 256x128 or, in a pair, 128x128} FP8 tiles,
 //               128-byte swizzled, either K-major or MN-major (transposed operands need no copy).
-//   warp 1      MMA issuer (one lane): 4 x tcgen05.mma (M128 N256 K32) per stage.  With blockwise
+//   warp 1      MMA issuer (one lane; in a pair the first CTA's, for both): 4 x tcgen05.mma (N256 K32) per stage.  With blockwise
 //               scales every 128-K block goes to one of two 256-column TMEM buffers with the
 //               accumulate flag cleared, so each buffer holds one *partial* product.
 //   warp 2      allocates / frees the 512 TMEM columns.
@@ -30,15 +33,20 @@ constexpr int kMaxAccBufs = 4;
 // 256-column TMEM buffers, 3 stages of 48 KiB.  (192- and 128-wide tiles were built and measured
 // slower on every shape -- 8192^3 blockwise: 2044 TFLOP/s at 256, 1558 at 192 with twelve promotion
 // warps, 1349 at 128 -- and are not compiled into the library.)
-// DEEP = 1 trades the output staging buffer for one more pipeline stage (plain stores in the epilogue).
-template <int BN, int DEEP> struct Geo {
-    static_assert(BN == 256, "only the 256-wide tile is built");
+// DEEP = 1 trades the output staging buffer for more pipeline stages (plain stores in the epilogue).
+//
+// CTAS = 2.  What bounds the one-CTA tile once the scales are applied at the end is its shared memory: a 128-wide
+// contraction block (8.4 MFLOP, 512 clocks of tensor pipe) writes and reads 48 KiB, 768 clocks at 128 bytes each; measured
+// 855.  In a pair each CTA moves 32 KiB for the same work, because the tensor cores of both SMs read both halves of B:
+// measured 730.
+template <int BN, int DEEP, int CTAS> struct Geo {
+    static_assert(BN == 256 && !(DEEP && CTAS == 2), "only these tiles are built");
     static constexpr int kSliceCols   = 128;                        // columns owned by one promotion warp
     static constexpr int kEpiWarps    = 4 * (BN / kSliceCols);      // 8
     static constexpr int kThreads     = 128 + 32 * kEpiWarps;
-    static constexpr int kBBytes      = BN * BK;
+    static constexpr int kBBytes      = BN * BK / CTAS;
     static constexpr int kStageBytes  = kABytes + kBBytes;
-    static constexpr int kStages      = 3 + DEEP;
+    static constexpr int kStages      = CTAS == 2 ? 4 : 3 + DEEP;
     static constexpr int kAccBufs     = 512 / BN;
     static constexpr int kChunks      = kSliceCols / 32;            // 32-column TMEM loads per partial
     static constexpr int kWarpCBytes  = 32 * kSliceCols * 2;        // staging of one warp's 32-row slab (16-bit out)
@@ -72,7 +80,10 @@ struct GemmArgs {
     uint32_t idesc;
     int M, N, K, G;
     int bn; // tile width the kernel was instantiated with
-    int deep; // 1: four-stage variant without output staging
+    int bm; // tile height: 128 per CTA of the tile
+    int ctas; // CTAs that share a tile (1 or 2)
+    int relay; // pairs, unpadded variable-K groups: the second CTA clears its own out-of-group rows and reports its stages
+    int deep; // 1: variant without output staging
     int tiles_n;
     const int64_t *group_offs;
     void *c;
@@ -97,6 +108,27 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// the same address in the shared memory of CTA `rank` of this cluster
+__device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+// Arrival on a barrier of the pair's other CTA.  What it hands over is tensor memory whose reads have completed
+// (tcgen05.wait::ld) or shared memory already fenced to the async proxy, so the default scope is enough; a release
+// at cluster scope waits for every outstanding access of the thread and tripled the time of the per-block modes.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_cta_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
 __device__ __forceinline__ uint32_t mbar_try(uint32_t bar, uint32_t parity) {
     uint32_t ok;
@@ -129,6 +161,15 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *tm,
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, "
                  "%5}], [%2];" ::"r"(dst),
                  "l"(tm), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+                 : "memory");
+}
+
+// the same into this CTA's shared memory, with the barrier in either CTA of the pair (a shared::cluster address)
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap *tm, uint32_t cluster_bar, int c0, int c1,
+                                                 int c2) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, "
+                 "{%3, %4, %5}], [%2];" ::"r"(dst),
+                 "l"(tm), "r"(cluster_bar), "r"(c0), "r"(c1), "r"(c2)
                  : "memory");
 }
 
@@ -168,12 +209,20 @@ __device__ __forceinline__ void cp_async_arrive_on(uint32_t bar) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+template <int CTAS = 1>
 __device__ __forceinline__ void tc_mma_f8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                           uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-                 "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-                 : "memory");
+    if constexpr (CTAS == 2) {
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                     "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+                     "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+                     : "memory");
+    } else {
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                     "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+                     "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+                     : "memory");
+    }
 }
 // block-scaled FP8 MMA: one E8M0 scale per 32 contraction elements of every A row and B row, read from
 // tensor memory; the byte of the 32-bit scale cell to use is part of the instruction descriptor
@@ -188,7 +237,14 @@ __device__ __forceinline__ void tc_mma_mxf8(uint32_t d_tmem, uint64_t adesc, uin
 __device__ __forceinline__ void tc_cp_sf(uint32_t dst_tmem, uint64_t sdesc) {
     asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(dst_tmem), "l"(sdesc) : "memory");
 }
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
+// Arrives on `bar` once the MMAs issued so far have retired; a pair's issuer arrives on that barrier of both CTAs.
+template <int CTAS = 1> __device__ __forceinline__ void tc_commit(uint32_t bar) {
+    if constexpr (CTAS == 2) {
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+                     "h"((uint16_t) 3)
+                     : "memory");
+        return;
+    }
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                  : "memory");
 }
@@ -266,7 +322,7 @@ struct __align__(16) SharedCtl {
     int group_offs[kMaxGroups + 1]; // copy of the device offsets: the schedule never waits on global memory
 };
 
-// Walks the tiles blockIdx.x, blockIdx.x + gridDim.x, ... of one CTA.  The linear index is split
+// Walks the tiles u, u + units, ... of one CTA or pair (u of units).  The linear index is split
 // into its coordinates once, with divisions, in the constructor; every later tile is reached by
 // adding the (pre-split) grid stride and carrying, because each role warp pays for the walk on its
 // critical path once per tile and short-K tiles (wgrad) last only a few thousand cycles.
@@ -277,7 +333,7 @@ struct Schedule {
     int p0, p1, p2; // dense: (band, index in band, -); grouped rows: (m-tile, n-tile, group cursor);
                     // grouped variable-K: (group, m-tile, n-tile)
 
-    __device__ Schedule(const GemmArgs &args, const SharedCtl *c) : a(args), ctl(c), lin(blockIdx.x) {
+    __device__ Schedule(const GemmArgs &args, const SharedCtl *c) : a(args), ctl(c), lin(blockIdx.x / args.ctas) {
         p0 = p1 = p2 = 0;
         if (lin >= ctl->total_tiles) return;
         if (a.kind == kKindDense) {
@@ -288,7 +344,7 @@ struct Schedule {
             p0 = lin / a.tiles_n;
             p1 = lin - p0 * a.tiles_n;
         } else {
-            const int per_g = ((a.M + BM - 1) / BM) * a.tiles_n;
+            const int per_g = ((a.M + a.bm - 1) / a.bm) * a.tiles_n;
             p0          = lin / per_g;
             const int r = lin - p0 * per_g;
             p1 = r / a.tiles_n;
@@ -299,7 +355,7 @@ struct Schedule {
     // Emits the current tile and steps to the CTA's next one; false when the CTA has no tile left.
     __device__ bool get(Tile &o) {
         if (lin >= ctl->total_tiles) return false;
-        const int step = gridDim.x, tiles_m = (a.M + BM - 1) / BM;
+        const int step = gridDim.x / a.ctas, tiles_m = (a.M + a.bm - 1) / a.bm;
         const int *offs = ctl->group_offs;
         if (a.kind == kKindDense) {
             // bands of 8 row-tiles, rows fastest inside a band: neighbouring CTAs share B columns
@@ -314,7 +370,7 @@ struct Schedule {
             }
             const int nt = rows == 8 ? (p1 >> 3) : p1 / rows;
             const int mt = 8 * p0 + (p1 - nt * rows);
-            o.m0 = mt * BM; o.m_end = a.M; o.n0 = nt * a.bn; o.g = 0; o.k_row0 = 0;
+            o.m0 = mt * a.bm; o.m_end = a.M; o.n0 = nt * a.bn; o.g = 0; o.k_row0 = 0;
             o.num_kb = (a.K + BK - 1) / BK; o.k_tail = 0;
             p1 += step;
         } else if (a.kind == kKindGroupedRows) {
@@ -322,14 +378,14 @@ struct Schedule {
             while (tile_prefix[p2 + 1] <= p0) ++p2;
             const int g  = p2;
             const int lo = offs[g], hi = offs[g + 1];
-            o.m0 = lo + (p0 - tile_prefix[g]) * BM; o.m_end = hi; o.n0 = p1 * a.bn; o.g = g;
+            o.m0 = lo + (p0 - tile_prefix[g]) * a.bm; o.m_end = hi; o.n0 = p1 * a.bn; o.g = g;
             o.k_row0 = 0; o.num_kb = (a.K + BK - 1) / BK; o.k_tail = 0;
             p1 += ctl->sched_rem;
             p0 += ctl->sched_q;
             if (p1 >= a.tiles_n) { p1 -= a.tiles_n; ++p0; }
         } else {
             const int lo = offs[p0], hi = offs[p0 + 1];
-            o.m0 = p1 * BM; o.m_end = a.M; o.n0 = p2 * a.bn; o.g = p0; o.k_row0 = lo;
+            o.m0 = p1 * a.bm; o.m_end = a.M; o.n0 = p2 * a.bn; o.g = p0; o.k_row0 = lo;
             o.num_kb = (hi - lo + BK - 1) / BK;
             o.k_tail = (hi - lo) % BK;
             p2 += ctl->sched_rem;
@@ -392,9 +448,22 @@ template <> struct Pack8<float> {
 };
 
 
-template <int SCALE, typename OutT, int BN, int DEEP>
-__global__ void __launch_bounds__(Geo<BN, DEEP>::kThreads, 1) fp8_gemm_kernel(const __grid_constant__ GemmArgs args) {
-    using G_ = Geo<BN, DEEP>;
+// The last block of an unpadded variable-K group reaches into the next group's rows (or past the last group): clear
+// those contraction rows in both MN-major operand tiles, so that whatever bytes lie there -- FP8 NaN patterns
+// included -- add nothing.  A contraction row is 128 bytes in the A tile and in each 128-column part of the B tile;
+// the swizzle only permutes bytes inside a row.  One warp.
+template <int B_PARTS> __device__ __forceinline__ void clear_tail_rows(uint8_t *a_tile, int k_tail, int lane) {
+    for (int off = k_tail * 128 + lane * 16; off < kABytes; off += 32 * 16) {
+#pragma unroll
+        for (int p = 0; p <= B_PARTS; ++p) *reinterpret_cast<uint4 *>(a_tile + p * 16384 + off) = make_uint4(0, 0, 0, 0);
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
+template <int SCALE, typename OutT, int BN, int DEEP, int CTAS>
+__global__ void __launch_bounds__(Geo<BN, DEEP, CTAS>::kThreads, 1) fp8_gemm_kernel(const __grid_constant__ GemmArgs args) {
+    using G_ = Geo<BN, DEEP, CTAS>;
+    static_assert(CTAS == 1 || SCALE == kScaleTensor || SCALE == kScaleRow, "block scales run one CTA per tile");
     constexpr int kStages = G_::kStages, kStageBytes = G_::kStageBytes, kThreads = G_::kThreads;
     constexpr int kAccBufs = (SCALE == kScaleMX) ? 1 : G_::kAccBufs, kWgCols = G_::kSliceCols, kChunks = G_::kChunks;
     constexpr int kCStageBytes = G_::kCStageBytes, kEpiWarps = G_::kEpiWarps;
@@ -406,17 +475,20 @@ __global__ void __launch_bounds__(Geo<BN, DEEP>::kThreads, 1) fp8_gemm_kernel(co
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t smem_base = smem_u32(smem);
+    const int rank     = CTAS == 2 ? (int) cluster_cta_rank() : 0; // this CTA's half of the tile
+    const bool leader  = rank == 0;
+    const bool relayed = CTAS == 2 && args.relay;
     constexpr bool kPerBlock = (SCALE == kScaleBlock2D || SCALE == kScaleBlock1D);
 
     // ---- set-up: barriers, tile table, tensor memory -------------------------------------------
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
-            mbar_init(smem_u32(&ctl->full[s]), 1);
+            mbar_init(smem_u32(&ctl->full[s]), relayed && leader ? 2 : 1);
             mbar_init(smem_u32(&ctl->empty[s]), 1);
         }
         for (int b = 0; b < kAccBufs; ++b) {
             mbar_init(smem_u32(&ctl->tmem_full[b]), 1);
-            mbar_init(smem_u32(&ctl->tmem_empty[b]), kEpiWarps); // one arrival per promotion warp
+            mbar_init(smem_u32(&ctl->tmem_empty[b]), CTAS * kEpiWarps); // one arrival per promotion warp
         }
         for (int b = 0; b < kScaleSlots; ++b) {
             mbar_init(smem_u32(&ctl->sc_full[b]), 32);         // every loader lane, after its own copies
@@ -433,20 +505,20 @@ __global__ void __launch_bounds__(Geo<BN, DEEP>::kThreads, 1) fp8_gemm_kernel(co
     }
     if (threadIdx.x == 32) {
         ctl->sf_batches_done = 0;
-        ctl->sched_q   = (int) gridDim.x / args.tiles_n;
-        ctl->sched_rem = (int) gridDim.x % args.tiles_n;
+        ctl->sched_q   = (int) (gridDim.x / CTAS) / args.tiles_n;
+        ctl->sched_rem = (int) (gridDim.x / CTAS) % args.tiles_n;
     }
     if (args.kind != kKindDense) {
         for (int g = threadIdx.x; g <= args.G; g += kThreads) ctl->group_offs[g] = (int) args.group_offs[g];
     }
     if (args.kind == kKindGroupedRows) {
-        // cumulative 128-row tiles per group; one warp scans (G <= kMaxGroups, checked on the host)
+        // cumulative row tiles per group; one warp scans (G <= kMaxGroups, checked on the host)
         if (warp == 3) {
             int run = 0;
             for (int base = 0; base < args.G; base += 32) {
                 const int g = base + lane;
                 int cnt     = 0;
-                if (g < args.G) cnt = (int) ((args.group_offs[g + 1] - args.group_offs[g] + BM - 1) / BM);
+                if (g < args.G) cnt = (int) ((args.group_offs[g + 1] - args.group_offs[g] + CTAS * BM - 1) / (CTAS * BM));
                 int inc = cnt;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
@@ -462,17 +534,25 @@ __global__ void __launch_bounds__(Geo<BN, DEEP>::kThreads, 1) fp8_gemm_kernel(co
             }
         }
     } else if (threadIdx.x == 0) {
-        const int tiles_m = (args.M + BM - 1) / BM;
+        const int tiles_m = (args.M + CTAS * BM - 1) / (CTAS * BM);
         ctl->total_tiles  = (args.kind == kKindDense ? 1 : args.G) * tiles_m * args.tiles_n;
     }
     if (warp == 2) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
-                         smem_u32(&ctl->tmem_base))
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if constexpr (CTAS == 2) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+                             smem_u32(&ctl->tmem_base))
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+                             smem_u32(&ctl->tmem_base))
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     tc_fence_before();
     __syncthreads();
+    if constexpr (CTAS == 2) cluster_sync(); // the other CTA's barriers are initialised too
     tc_fence_after();
     const uint32_t tmem_base = ctl->tmem_base;
 
@@ -480,10 +560,12 @@ __global__ void __launch_bounds__(Geo<BN, DEEP>::kThreads, 1) fp8_gemm_kernel(co
         // register split between the helper warpgroup and the two promotion warpgroups: the 1-D x 1-D
         // promotion needs every register it can get, the other modes leave more to the MMA issuer
         // (in MX mode the scale loader keeps four blocks of scale words in registers and the epilogue holds no
-        // promotion state, so the split moves the other way)
+        // promotion state, so the split moves the other way).  Neither side may spill in a loop: with the shared memory all
+        // taken the L1 is tiny and a spilled register comes back from L2.
         if constexpr (SCALE == kScaleBlock1D) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+        else if constexpr (SCALE == kScaleBlock2D) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
         else if constexpr (SCALE == kScaleMX) asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
-        else asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+        else asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
         if (warp == 0 && lane == 0) {
             // ================= TMA producer =================
             Schedule sched(args, ctl);
@@ -497,9 +579,26 @@ __global__ void __launch_bounds__(Geo<BN, DEEP>::kThreads, 1) fp8_gemm_kernel(co
                     const uint32_t ph = (it / kStages) & 1;
                     if (!mbar_wait(smem_u32(&ctl->empty[s]), ph ^ 1)) { ok = false; break; }
                     const uint32_t full = smem_u32(&ctl->full[s]);
-                    mbar_expect_tx(full, kStageBytes);
                     const uint32_t sa = smem_base + s * kStageBytes, sb = sa + kABytes;
                     const int k = t.k_row0 + kb * BK;
+                    if constexpr (CTAS == 2) {
+                        // Both CTAs' copies complete on the first CTA's barrier, except where the second relays.  A
+                        // half of A that holds no row of the tile is not fetched: its products are never read.
+                        const int m0 = t.m0 + rank * BM, n0 = t.n0 + rank * (BN / 2);
+                        const bool has_a = m0 < t.m_end;
+                        uint32_t bar     = full;
+                        if (relayed) mbar_expect_tx(full, has_a ? kStageBytes : kStageBytes - kABytes);
+                        else if (leader) mbar_expect_tx(full, m0 + BM < t.m_end ? 2 * kStageBytes : 2 * kStageBytes - kABytes);
+                        if (!relayed) bar = map_to_cta(full, 0);
+                        if (has_a) {
+                            if (args.a_mn) tma_load_3d_pair(sa, &args.tm_a, bar, m0, k, 0);
+                            else           tma_load_3d_pair(sa, &args.tm_a, bar, k, m0, 0);
+                        }
+                        if (args.b_mn) tma_load_3d_pair(sb, &args.tm_b, bar, n0, k, gb);
+                        else           tma_load_3d_pair(sb, &args.tm_b, bar, k, n0, gb);
+                        continue;
+                    }
+                    mbar_expect_tx(full, kStageBytes);
                     if (args.a_mn) tma_load_3d(sa, &args.tm_a, full, t.m0, k, 0);
                     else           tma_load_3d(sa, &args.tm_a, full, k, t.m0, 0);
                     if (args.b_mn) {
@@ -512,12 +611,33 @@ __global__ void __launch_bounds__(Geo<BN, DEEP>::kThreads, 1) fp8_gemm_kernel(co
             }
             if (!ok) {
                 atomicExch(&g_gemm_status, 1);
-                // let the copies already issued land before the CTA releases its shared memory
+                // let the copies already issued land before the CTA releases its shared memory (a pair's second CTA
+                // finds its copies' barrier in the first; the pair leaves together, after the first has waited)
+                if (CTAS == 2 && !leader && !relayed) it = 0;
                 const uint32_t back = it < (uint32_t) kStages ? it : (uint32_t) kStages;
                 for (uint32_t j = 1; j <= back; ++j) {
                     const uint32_t q = it - j;
                     mbar_wait(smem_u32(&ctl->full[q % kStages]), (q / kStages) & 1);
                 }
+            }
+        } else if (warp == 1 && !leader) {
+            // ================= second CTA of a pair: reports its stages where they need work first =================
+            if (relayed) {
+                Schedule sched(args, ctl);
+                Tile t;
+                uint32_t it = 0;
+                bool ok     = true;
+                while (ok && sched.get(t)) {
+                    for (int kb = 0; kb < t.num_kb; ++kb, ++it) {
+                        const int s = it % kStages;
+                        if (!mbar_wait(smem_u32(&ctl->full[s]), (it / kStages) & 1)) { ok = false; break; }
+                        if (t.k_tail != 0 && kb == t.num_kb - 1)
+                            clear_tail_rows<G_::kBBytes / 16384>(smem + s * kStageBytes, t.k_tail, lane);
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&ctl->full[s]), 0));
+                    }
+                }
+                if (!ok && lane == 0) atomicExch(&g_gemm_status, 2);
             }
         } else if (warp == 1) {
             // ================= MMA issuer (whole warp walks the schedule, lane 0 issues) =================
@@ -526,7 +646,7 @@ __global__ void __launch_bounds__(Geo<BN, DEEP>::kThreads, 1) fp8_gemm_kernel(co
             uint32_t it = 0, acc_it = 0;
             bool ok     = true;
             const uint32_t a_lbo = 0, a_sbo = 1024, a_step = args.a_mn ? 4096u : 32u;
-            const uint32_t b_lbo = args.b_mn ? 16384u : 0u, b_sbo = 1024;
+            const uint32_t b_lbo = args.b_mn && CTAS == 1 ? 16384u : 0u, b_sbo = 1024;
             const uint32_t b_step = args.b_mn ? 4096u : 32u;
             while (ok && sched.get(t)) {
                 for (int kb = 0; kb < t.num_kb; ++kb, ++it) {
@@ -543,19 +663,7 @@ __global__ void __launch_bounds__(Geo<BN, DEEP>::kThreads, 1) fp8_gemm_kernel(co
                         if (!mbar_wait(smem_u32(&ctl->sc_full[slot]), (it / kScaleSlots) & 1)) { ok = false; break; }
                     }
                     uint8_t *a_tile = smem + s * kStageBytes;
-                    if (t.k_tail != 0 && kb == t.num_kb - 1) {
-                        // The last block of an unpadded group reaches into the next group's rows (or
-                        // past the last group): clear those contraction rows in both MN-major operand
-                        // tiles, so that whatever bytes lie there -- FP8 NaN patterns included -- add
-                        // nothing.  A contraction row is 128 bytes in the A tile and in each of the two
-                        // 128-column halves of the B tile; the swizzle only permutes bytes inside a row.
-                        for (int off = t.k_tail * 128 + lane * 16; off < kABytes; off += 32 * 16) {
-                            *reinterpret_cast<uint4 *>(a_tile + off)                   = make_uint4(0, 0, 0, 0);
-                            *reinterpret_cast<uint4 *>(a_tile + kABytes + off)         = make_uint4(0, 0, 0, 0);
-                            *reinterpret_cast<uint4 *>(a_tile + kABytes + 16384 + off) = make_uint4(0, 0, 0, 0);
-                        }
-                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    }
+                    if (t.k_tail != 0 && kb == t.num_kb - 1) clear_tail_rows<G_::kBBytes / 16384>(a_tile, t.k_tail, lane);
                     __syncwarp();
                     tc_fence_after();
                     if (lane == 0) {
@@ -583,15 +691,15 @@ __global__ void __launch_bounds__(Geo<BN, DEEP>::kThreads, 1) fp8_gemm_kernel(co
 #pragma unroll
                             for (int j = 0; j < BK / 32; ++j) {
                                 const uint32_t accumulate = (j > 0 || !new_acc) ? 1u : 0u;
-                                tc_mma_f8(d, ad + (uint64_t) ((a_step * j) >> 4), bd + (uint64_t) ((b_step * j) >> 4),
-                                          args.idesc, accumulate);
+                                tc_mma_f8<CTAS>(d, ad + (uint64_t) ((a_step * j) >> 4), bd + (uint64_t) ((b_step * j) >> 4),
+                                                args.idesc, accumulate);
                             }
                         }
-                        tc_commit(smem_u32(&ctl->empty[s])); // stage reusable once these MMAs retire
+                        tc_commit<CTAS>(smem_u32(&ctl->empty[s])); // stage reusable once these MMAs retire
                     }
                     const bool last = kPerBlock || kb == t.num_kb - 1;
                     if (last) {
-                        if (lane == 0) tc_commit(smem_u32(&ctl->tmem_full[buf]));
+                        if (lane == 0) tc_commit<CTAS>(smem_u32(&ctl->tmem_full[buf]));
                         ++acc_it;
                     }
                 }
@@ -742,8 +850,9 @@ __global__ void __launch_bounds__(Geo<BN, DEEP>::kThreads, 1) fp8_gemm_kernel(co
         }
     } else {
         if constexpr (SCALE == kScaleBlock1D) asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
+        else if constexpr (SCALE == kScaleBlock2D) asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
         else if constexpr (SCALE == kScaleMX) asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
-        else asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+        else asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
         // ================= promotion + epilogue warpgroups =================
         const int wg   = (warp - 4) >> 2;         // column slice of the tile this warp owns
         const int quad = warp & 3;                // TMEM lane quadrant this warp may read
@@ -774,11 +883,28 @@ __global__ void __launch_bounds__(Geo<BN, DEEP>::kThreads, 1) fp8_gemm_kernel(co
         float acc[kWgCols];
         while (ok && sched.get(t)) {
             const int gb      = (args.kind == kKindGroupedRows) ? t.g : 0;
+            if constexpr (CTAS == 2) t.m0 += rank * BM; // this CTA's rows (none, where the group ends before them)
             const int row     = t.m0 + row_in_tile;
             const int col0    = t.n0 + wg * kWgCols;
             const int segs    = kPerBlock ? t.num_kb : (t.num_kb > 0 ? 1 : 0);
 #pragma unroll
             for (int j = 0; j < kWgCols; ++j) acc[j] = 0.0f;
+
+            // tensorwise / rowwise scales; a warp's column scales wait in its part of the (otherwise unused) ring, fetched
+            // before the tile's products are awaited: 128 loads per thread at the end of the tile made the
+            // rowwise 8192^3 18 % slower than the tensorwise one
+            float *my_cols = &ctl->scale_ring[(warp - 4) * kWgCols];
+            float sa       = 1.0f;
+            if constexpr (SCALE == kScaleTensor) sa = args.a_scale[0] * args.b_scale[0];
+            if constexpr (SCALE == kScaleRow) {
+                sa = args.a_scale[(int64_t) min(row, t.m_end - 1) * args.as_m];
+                const float *bs = args.b_scale + (int64_t) gb * args.bs_g;
+                __syncwarp(); // the previous tile's scales have been read
+#pragma unroll
+                for (int i = 0; i < kWgCols / 32; ++i)
+                    my_cols[i * 32 + lane] = bs[(int64_t) min(col0 + i * 32 + lane, args.N - 1) * args.bs_n];
+                __syncwarp();
+            }
 
             // 1-D x 2-D block scales: each thread fetches its two scalars two contraction blocks
             // ahead of their use
@@ -849,7 +975,10 @@ __global__ void __launch_bounds__(Geo<BN, DEEP>::kThreads, 1) fp8_gemm_kernel(co
                 tc_wait_ld();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&ctl->tmem_empty[buf])); // buffer may be overwritten now
+                if (lane == 0) { // buffer may be overwritten now
+                    if constexpr (CTAS == 2) mbar_arrive_cluster(map_to_cta(smem_u32(&ctl->tmem_empty[buf]), 0));
+                    else mbar_arrive(smem_u32(&ctl->tmem_empty[buf]));
+                }
                 PTB_PROMOTE(v0, 2)
                 PTB_PROMOTE(v1, 3)
 #undef PTB_PROMOTE
@@ -861,18 +990,15 @@ __global__ void __launch_bounds__(Geo<BN, DEEP>::kThreads, 1) fp8_gemm_kernel(co
             if (!ok) break;
 
             // ---- scale (tensorwise / rowwise), convert and store ---------------------------------
-            float sa = 1.0f;
-            if constexpr (SCALE == kScaleTensor) sa = args.a_scale[0] * args.b_scale[0];
-            if constexpr (SCALE == kScaleRow) sa = args.a_scale[(int64_t) min(row, t.m_end - 1) * args.as_m];
-            if constexpr (SCALE == kScaleTensor || SCALE == kScaleRow) {
+            if constexpr (SCALE == kScaleTensor) {
 #pragma unroll
-                for (int j = 0; j < kWgCols; ++j) {
-                    float s = sa;
-                    if constexpr (SCALE == kScaleRow) {
-                        const int c = col0 + j;
-                        s = sa * ((c < args.N) ? args.b_scale[(int64_t) gb * args.bs_g + (int64_t) c * args.bs_n] : 0.0f);
-                    }
-                    acc[j] *= s;
+                for (int j = 0; j < kWgCols; ++j) acc[j] *= sa;
+            }
+            if constexpr (SCALE == kScaleRow) {
+#pragma unroll
+                for (int j = 0; j < kWgCols; j += 4) {
+                    const float4 c4 = *reinterpret_cast<const float4 *>(my_cols + j);
+                    acc[j] *= sa * c4.x; acc[j + 1] *= sa * c4.y; acc[j + 2] *= sa * c4.z; acc[j + 3] *= sa * c4.w;
                 }
             }
             const int warp_row0 = t.m0 + quad * 32;
@@ -924,9 +1050,12 @@ __global__ void __launch_bounds__(Geo<BN, DEEP>::kThreads, 1) fp8_gemm_kernel(co
     // ---- teardown -----------------------------------------------------------------------------------
     tc_fence_before();
     __syncthreads();
+    // neither CTA of a pair leaves while the other may still signal its barriers or read its operands
+    if constexpr (CTAS == 2) cluster_sync();
     if (warp == 2) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
+        if constexpr (CTAS == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
     }
 }
 
@@ -1005,7 +1134,7 @@ int make_c_map(CUtensorMap *tm, int *ok, void *c, int out_dtype, uint64_t cols, 
     return 0;
 }
 
-uint32_t make_idesc(int a_dtype, int b_dtype, int a_mn, int b_mn, int BN) {
+uint32_t make_idesc(int a_dtype, int b_dtype, int a_mn, int b_mn, int BN, int ctas = 1) {
     uint32_t d = 0;
     d |= 1u << 4;                                    // D format fp32
     d |= (a_dtype == PTB_E5M2 ? 1u : 0u) << 7;       // A format
@@ -1013,7 +1142,7 @@ uint32_t make_idesc(int a_dtype, int b_dtype, int a_mn, int b_mn, int BN) {
     d |= (uint32_t) (a_mn ? 1 : 0) << 15;            // A major
     d |= (uint32_t) (b_mn ? 1 : 0) << 16;            // B major
     d |= (uint32_t) (BN >> 3) << 17;                 // N
-    d |= (uint32_t) (BM >> 4) << 24;                 // M
+    d |= (uint32_t) (ctas * BM >> 4) << 24;          // M
     return d;
 }
 
@@ -1029,30 +1158,46 @@ uint32_t make_idesc_mx(int a_dtype, int b_dtype, int BN) {
     return d;
 }
 
-template <int BN, int DEEP> constexpr size_t smem_bytes() {
-    return 1024 + (size_t) Geo<BN, DEEP>::kStages * Geo<BN, DEEP>::kStageBytes + Geo<BN, DEEP>::kCStageBytes +
-           sizeof(SharedCtl);
+template <int BN, int DEEP, int CTAS> constexpr size_t smem_bytes() {
+    using G_ = Geo<BN, DEEP, CTAS>;
+    return 1024 + (size_t) G_::kStages * G_::kStageBytes + G_::kCStageBytes + sizeof(SharedCtl);
 }
-static_assert(smem_bytes<256, 0>() <= 232448 && smem_bytes<256, 1>() <= 232448,
+static_assert(smem_bytes<256, 0, 1>() <= 232448 && smem_bytes<256, 1, 1>() <= 232448 && smem_bytes<256, 0, 2>() <= 232448,
               "shared memory budget of one CTA exceeded");
 
-template <int SCALE, typename OutT, int BN, int DEEP> int launch_bn(const GemmArgs &args, int grid, cudaStream_t st) {
+template <int SCALE, typename OutT, int BN, int DEEP, int CTAS> int launch_bn(const GemmArgs &args, int grid, cudaStream_t st) {
     static bool configured[64] = {}; // per device; the attribute set is idempotent, a race only repeats it
-    constexpr size_t kSmemBytes = smem_bytes<BN, DEEP>();
-    auto kfn = fp8_gemm_kernel<SCALE, OutT, BN, DEEP>;
+    constexpr size_t kSmemBytes = smem_bytes<BN, DEEP, CTAS>();
+    auto kfn = fp8_gemm_kernel<SCALE, OutT, BN, DEEP, CTAS>;
     int dev  = 0;
     PTB_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || !configured[dev]) {
         PTB_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kSmemBytes));
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    kfn<<<grid, Geo<BN, DEEP>::kThreads, kSmemBytes, st>>>(args);
+    if constexpr (CTAS == 2) {
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute attr{};
+        attr.id               = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = 2;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.gridDim = dim3((unsigned) (grid & ~1)); cfg.blockDim = dim3(Geo<BN, DEEP, CTAS>::kThreads);
+        cfg.dynamicSmemBytes = kSmemBytes; cfg.stream = st; cfg.attrs = &attr; cfg.numAttrs = 1;
+        PTB_CUDA(cudaLaunchKernelEx(&cfg, kfn, args));
+    } else {
+        kfn<<<grid, Geo<BN, DEEP, CTAS>::kThreads, kSmemBytes, st>>>(args);
+    }
     PTB_LAUNCH_CHECK("fp8_gemm_kernel");
     return 0;
 }
 
 template <int SCALE, typename OutT> int launch_one(const GemmArgs &args, int grid, cudaStream_t st) {
-    return args.deep ? launch_bn<SCALE, OutT, 256, 1>(args, grid, st) : launch_bn<SCALE, OutT, 256, 0>(args, grid, st);
+    constexpr bool kCanDeep = SCALE == kScaleTensor || SCALE == kScaleRow;
+    if constexpr (kCanDeep) {
+        if (args.ctas == 2) return launch_bn<SCALE, OutT, 256, 0, 2>(args, grid, st);
+        if (args.deep) return launch_bn<SCALE, OutT, 256, 1, 1>(args, grid, st);
+    }
+    return launch_bn<SCALE, OutT, 256, 0, 1>(args, grid, st);
 }
 
 template <int SCALE> int launch_scale(const GemmArgs &args, int out_dtype, int grid, cudaStream_t st) {
@@ -1064,19 +1209,38 @@ template <int SCALE> int launch_scale(const GemmArgs &args, int out_dtype, int g
     }
 }
 
-#ifndef PTB_MX_DEEP
-#define PTB_MX_DEEP 0
-#endif
-
-int launch_gemm(GemmArgs &args, int scale_mode, int out_dtype, int num_sms, cudaStream_t st) {
-    // Tensorwise / rowwise scales keep the whole K loop in TMEM, so the epilogue is rare: spend the
-    // staging buffer on a fourth pipeline stage instead (measured +8 % on 8192^3).
-    args.deep = ((scale_mode == kScaleTensor || scale_mode == kScaleRow || (scale_mode == kScaleMX && PTB_MX_DEEP)) &&
-                 args.kind == kKindDense) ? 1 : 0;
+// CTAs of a persistent launch: one per SM, or the caller's cap
+int persistent_grid(int num_sms, int *grid) {
     int dev = 0, sms = 0;
     PTB_CUDA(cudaGetDevice(&dev));
     PTB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    int grid = (num_sms > 0 && num_sms < sms) ? num_sms : sms;
+    *grid = (num_sms > 0 && num_sms < sms) ? num_sms : sms;
+    return 0;
+}
+
+constexpr int kTileN = 256;
+
+// CTAs per tile.  Only tensorwise and rowwise scales run in pairs: with block scales the promotion warps set the pace
+// and a second CTA's hand-shakes slow them (8192^3 NT, 128 x 128 weight blocks: 0.54 ms alone, 0.66 in pairs).  A contraction
+// block of the one-CTA tile takes 855 clocks (48 KiB in and 48 KiB out of a 128 B/clock shared memory), of the
+// pair's 730, so per SM a wave of pairs counts 6 / 7 of a wave of single tiles; where the 256-row tiles' padding or
+// the last wave costs more than that, tiles stay single.  8192^3: tensorwise 424 -> 404 us, rowwise 498 -> 462 us.
+int dense_ctas(int mode, int64_t M, int64_t N, int grid) {
+    if ((mode != kScaleTensor && mode != kScaleRow) || grid < 2) return 1;
+    const int64_t tn = cdiv<int64_t>(N, kTileN);
+    return cdiv<int64_t>(cdiv<int64_t>(M, 2 * BM) * tn, grid / 2) * 6 <= cdiv<int64_t>(cdiv<int64_t>(M, BM) * tn, grid) * 7 ? 2 : 1;
+}
+// Row groups: how many rows each group has is known on the device only.  With uneven groups of 256 rows on average the
+// 256-row tiles' padding eats the gain (log-normal loads: 317 single tiles against 2 x 198); from 384 on it does not.
+int grouped_ctas(int mode, int64_t rows, int64_t G, int grid) {
+    return (mode == kScaleTensor || mode == kScaleRow) && grid >= 2 && rows >= 384 * G ? 2 : 1;
+}
+
+int launch_gemm(GemmArgs &args, int scale_mode, int out_dtype, int grid, cudaStream_t st) {
+    // Tensorwise / rowwise scales keep the whole K loop in TMEM, so the epilogue is rare: spend the
+    // staging buffer on a fourth pipeline stage instead (measured +8 % on 8192^3).
+    // (A pair's stages are smaller: it has four beside the staging buffer.)
+    args.deep = (scale_mode == kScaleTensor || scale_mode == kScaleRow) && args.kind == kKindDense && args.ctas == 1 ? 1 : 0;
     switch (scale_mode) {
     case kScaleTensor: return launch_scale<kScaleTensor>(args, out_dtype, grid, st);
     case kScaleRow: return launch_scale<kScaleRow>(args, out_dtype, grid, st);
@@ -1087,7 +1251,12 @@ int launch_gemm(GemmArgs &args, int scale_mode, int out_dtype, int num_sms, cuda
     }
 }
 
-constexpr int kTileN = 256;
+// the fields every entry point derives from the number of CTAs per tile
+void set_tile(GemmArgs &g, int ctas) {
+    g.ctas = ctas;
+    g.bm   = ctas * BM;
+    g.bn   = kTileN;
+}
 
 int scale_mode_of(int granularity, int b_block_2d, int *mode) {
     switch (granularity) {
@@ -1145,17 +1314,21 @@ int ptb_gemm_fp8(const void *a, int a_dtype, int trans_a, int64_t lda, const voi
     if (rc) return rc;
     GemmArgs g{};
     const int BN = kTileN;
-    g.bn         = BN;
+    int grid = 0;
+    rc       = persistent_grid(num_sms, &grid);
+    if (rc) return rc;
+    const int ctas = dense_ctas(mode, M, N, grid);
+    set_tile(g, ctas);
     // A: [M,K] K-major, or [K,M] (trans_a) MN-major
     if (!trans_a) rc = make_map(&g.tm_a, a, (uint64_t) K, (uint64_t) M, 1, (uint64_t) lda, (uint64_t) lda * M, BM);
     else          rc = make_map(&g.tm_a, a, (uint64_t) M, (uint64_t) K, 1, (uint64_t) lda, (uint64_t) lda * K, BK);
     if (rc) return rc;
     // B: [N,K] (trans_b) K-major, or [K,N] MN-major
-    if (trans_b) rc = make_map(&g.tm_b, b, (uint64_t) K, (uint64_t) N, 1, (uint64_t) ldb, (uint64_t) ldb * N, BN);
+    if (trans_b) rc = make_map(&g.tm_b, b, (uint64_t) K, (uint64_t) N, 1, (uint64_t) ldb, (uint64_t) ldb * N, BN / ctas);
     else         rc = make_map(&g.tm_b, b, (uint64_t) N, (uint64_t) K, 1, (uint64_t) ldb, (uint64_t) ldb * K, BK);
     if (rc) return rc;
     g.kind = kKindDense; g.a_mn = trans_a ? 1 : 0; g.b_mn = trans_b ? 0 : 1;
-    g.idesc = make_idesc(a_dtype, b_dtype, g.a_mn, g.b_mn, BN);
+    g.idesc = make_idesc(a_dtype, b_dtype, g.a_mn, g.b_mn, BN, ctas);
     g.M = (int) M; g.N = (int) N; g.K = (int) K; g.G = 1;
     g.tiles_n = (int) cdiv<int64_t>(N, BN);
     g.c = c; g.ldc = ldc; g.c_group_stride = 0;
@@ -1163,7 +1336,7 @@ int ptb_gemm_fp8(const void *a, int a_dtype, int trans_a, int64_t lda, const voi
     if (rc) return rc;
     g.a_scale = a_scale; g.as_m = a_scale_stride_m; g.as_k = a_scale_stride_k;
     g.b_scale = b_scale; g.bs_g = 0; g.bs_n = b_scale_stride_n; g.bs_k = b_scale_stride_k;
-    return launch_gemm(g, mode, c_dtype, num_sms, (cudaStream_t) stream);
+    return launch_gemm(g, mode, c_dtype, grid, (cudaStream_t) stream);
 }
 
 int ptb_gemm_mxfp8(const void *a, int a_dtype, int64_t lda, const void *a_sf, int64_t a_sf_ld, const void *b, int b_dtype,
@@ -1181,7 +1354,7 @@ int ptb_gemm_mxfp8(const void *a, int a_dtype, int64_t lda, const void *a_sf, in
                 PTB_ERR_ALIGN, "gemm_mxfp8: scale rows must hold K/32 bytes, be 4-byte aligned and a multiple of 4 bytes apart");
     GemmArgs g{};
     const int BN = kTileN;
-    g.bn         = BN;
+    set_tile(g, 1);
     int rc = make_map(&g.tm_a, a, (uint64_t) K, (uint64_t) M, 1, (uint64_t) lda, (uint64_t) lda * M, BM);
     if (rc) return rc;
     rc = make_map(&g.tm_b, b, (uint64_t) K, (uint64_t) N, 1, (uint64_t) ldb, (uint64_t) ldb * N, BN);
@@ -1194,7 +1367,10 @@ int ptb_gemm_mxfp8(const void *a, int a_dtype, int64_t lda, const void *a_sf, in
     rc = make_c_map(&g.tm_c, &g.use_tma_store, c, c_dtype, (uint64_t) N, (uint64_t) M, 1, (uint64_t) ldc, 0);
     if (rc) return rc;
     g.a_sf = (const uint8_t *) a_sf; g.a_sf_ld = a_sf_ld; g.b_sf = (const uint8_t *) b_sf; g.b_sf_ld = b_sf_ld;
-    return launch_gemm(g, kScaleMX, c_dtype, num_sms, (cudaStream_t) stream);
+    int grid = 0;
+    rc       = persistent_grid(num_sms, &grid);
+    if (rc) return rc;
+    return launch_gemm(g, kScaleMX, c_dtype, grid, (cudaStream_t) stream);
 }
 
 int ptb_grouped_gemm_mxfp8(const void *a, int a_dtype, int64_t lda, const void *a_sf, int64_t a_sf_ld, const void *b,
@@ -1214,7 +1390,7 @@ int ptb_grouped_gemm_mxfp8(const void *a, int a_dtype, int64_t lda, const void *
                 PTB_ERR_ALIGN, "grouped_gemm_mxfp8: scale rows must hold K/32 bytes, be 4-byte aligned and a multiple of 4 apart");
     GemmArgs g{};
     const int BN = kTileN;
-    g.bn         = BN;
+    set_tile(g, 1);
     int rc = make_map(&g.tm_a, a, (uint64_t) K, (uint64_t) M_total, 1, (uint64_t) lda, (uint64_t) lda * M_total, BM);
     if (rc) return rc;
     rc = make_map(&g.tm_b, b, (uint64_t) K, (uint64_t) N, (uint64_t) G, (uint64_t) K, (uint64_t) K * N, BN);
@@ -1228,7 +1404,10 @@ int ptb_grouped_gemm_mxfp8(const void *a, int a_dtype, int64_t lda, const void *
     rc = make_c_map(&g.tm_c, &g.use_tma_store, out, out_dtype, (uint64_t) N, (uint64_t) M_total, 1, (uint64_t) ldc, 0);
     if (rc) return rc;
     g.a_sf = (const uint8_t *) a_sf; g.a_sf_ld = a_sf_ld; g.b_sf = (const uint8_t *) b_sf; g.b_sf_ld = K / 32;
-    return launch_gemm(g, kScaleMX, out_dtype, num_sms, (cudaStream_t) stream);
+    int grid = 0;
+    rc       = persistent_grid(num_sms, &grid);
+    if (rc) return rc;
+    return launch_gemm(g, kScaleMX, out_dtype, grid, (cudaStream_t) stream);
 }
 
 int ptb_grouped_gemm_mxfp8_variable_k(const void *lhs, int lhs_dtype, int64_t ld_lhs, const void *lhs_sf, int64_t lhs_sf_ld,
@@ -1250,7 +1429,7 @@ int ptb_grouped_gemm_mxfp8_variable_k(const void *lhs, int lhs_dtype, int64_t ld
                 PTB_ERR_ALIGN, "grouped_gemm_mxfp8_variable_k: scale rows must be 4-byte aligned and a multiple of 4 apart");
     GemmArgs g{};
     const int BN = kTileN;
-    g.bn         = BN;
+    set_tile(g, 1);
     const uint64_t r = rows_padded > 0 ? (uint64_t) rows_padded : 1;
     // both operands are transposed copies: [OUT_M, rows] and [OUT_N, rows], contraction axis contiguous
     int rc = make_map(&g.tm_a, lhs, r, (uint64_t) OUT_M, 1, (uint64_t) ld_lhs, (uint64_t) ld_lhs * OUT_M, BM);
@@ -1267,7 +1446,10 @@ int ptb_grouped_gemm_mxfp8_variable_k(const void *lhs, int lhs_dtype, int64_t ld
                     (uint64_t) OUT_N, (uint64_t) (OUT_M * OUT_N));
     if (rc) return rc;
     g.a_sf = (const uint8_t *) lhs_sf; g.a_sf_ld = lhs_sf_ld; g.b_sf = (const uint8_t *) rhs_sf; g.b_sf_ld = rhs_sf_ld;
-    return launch_gemm(g, kScaleMX, out_dtype, num_sms, (cudaStream_t) stream);
+    int grid = 0;
+    rc       = persistent_grid(num_sms, &grid);
+    if (rc) return rc;
+    return launch_gemm(g, kScaleMX, out_dtype, grid, (cudaStream_t) stream);
 }
 
 int ptb_grouped_gemm_fp8(const void *a, int a_dtype, int64_t lda, const void *b, int b_dtype, int trans_b, void *out,
@@ -1288,14 +1470,18 @@ int ptb_grouped_gemm_fp8(const void *a, int a_dtype, int64_t lda, const void *b,
     if (rc) return rc;
     GemmArgs g{};
     const int BN = kTileN;
-    g.bn         = BN;
+    int grid = 0;
+    rc       = persistent_grid(num_sms, &grid);
+    if (rc) return rc;
+    const int ctas = grouped_ctas(mode, M_total, G, grid);
+    set_tile(g, ctas);
     rc = make_map(&g.tm_a, a, (uint64_t) K, (uint64_t) M_total, 1, (uint64_t) lda, (uint64_t) lda * M_total, BM);
     if (rc) return rc;
-    if (trans_b) rc = make_map(&g.tm_b, b, (uint64_t) K, (uint64_t) N, (uint64_t) G, (uint64_t) K, (uint64_t) K * N, BN);
+    if (trans_b) rc = make_map(&g.tm_b, b, (uint64_t) K, (uint64_t) N, (uint64_t) G, (uint64_t) K, (uint64_t) K * N, BN / ctas);
     else         rc = make_map(&g.tm_b, b, (uint64_t) N, (uint64_t) K, (uint64_t) G, (uint64_t) N, (uint64_t) K * N, BK);
     if (rc) return rc;
     g.kind = kKindGroupedRows; g.a_mn = 0; g.b_mn = trans_b ? 0 : 1;
-    g.idesc = make_idesc(a_dtype, b_dtype, g.a_mn, g.b_mn, BN);
+    g.idesc = make_idesc(a_dtype, b_dtype, g.a_mn, g.b_mn, BN, ctas);
     g.M = (int) M_total; g.N = (int) N; g.K = (int) K; g.G = (int) G;
     g.tiles_n = (int) cdiv<int64_t>(N, BN);
     g.group_offs = group_offs;
@@ -1304,7 +1490,7 @@ int ptb_grouped_gemm_fp8(const void *a, int a_dtype, int64_t lda, const void *b,
     if (rc) return rc;
     g.a_scale = a_scale; g.as_m = a_scale_stride_m; g.as_k = a_scale_stride_k;
     g.b_scale = b_scale; g.bs_g = b_scale_stride_g; g.bs_n = b_scale_stride_n; g.bs_k = b_scale_stride_k;
-    return launch_gemm(g, mode, out_dtype, num_sms, (cudaStream_t) stream);
+    return launch_gemm(g, mode, out_dtype, grid, (cudaStream_t) stream);
 }
 
 int ptb_grouped_gemm_fp8_variable_k(const void *lhs, int lhs_dtype, int64_t ld_lhs, const void *rhs, int rhs_dtype,
@@ -1326,14 +1512,19 @@ int ptb_grouped_gemm_fp8_variable_k(const void *lhs, int lhs_dtype, int64_t ld_l
                 PTB_ERR_TOO_LARGE, "grouped_gemm_fp8_variable_k: problem too large");
     GemmArgs g{};
     const int BN = kTileN;
-    g.bn         = BN;
+    int grid = 0;
+    rc       = persistent_grid(num_sms, &grid);
+    if (rc) return rc;
+    const int ctas = (mode == kScaleTensor || mode == kScaleRow) && OUT_M > BM && grid >= 2 ? 2 : 1;
+    set_tile(g, ctas);
+    g.relay = mode != kScaleBlock1D; // unpadded groups: contraction rows past a group's end have to be cleared
     const uint64_t r = rows > 0 ? (uint64_t) rows : 1;
     rc = make_map(&g.tm_a, lhs, (uint64_t) OUT_M, r, 1, (uint64_t) ld_lhs, (uint64_t) ld_lhs * r, BK);
     if (rc) return rc;
     rc = make_map(&g.tm_b, rhs, (uint64_t) OUT_N, r, 1, (uint64_t) ld_rhs, (uint64_t) ld_rhs * r, BK);
     if (rc) return rc;
     g.kind = kKindGroupedK; g.a_mn = 1; g.b_mn = 1;
-    g.idesc = make_idesc(lhs_dtype, rhs_dtype, 1, 1, BN);
+    g.idesc = make_idesc(lhs_dtype, rhs_dtype, 1, 1, BN, ctas);
     g.M = (int) OUT_M; g.N = (int) OUT_N; g.K = (int) rows; g.G = (int) G;
     g.tiles_n = (int) cdiv<int64_t>(OUT_N, BN);
     g.group_offs = group_offs;
@@ -1348,14 +1539,10 @@ int ptb_grouped_gemm_fp8_variable_k(const void *lhs, int lhs_dtype, int64_t ld_l
         // blockwise wgrad on tile-aligned shapes: 256 x 128 paired tiles (see ptb_gemm_wgrad.cuh)
         g.bn = 128;
         g.idesc = make_idesc(lhs_dtype, rhs_dtype, 1, 1, 128);
-        int dev = 0, sms = 0;
-        PTB_CUDA(cudaGetDevice(&dev));
-        PTB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        const int grid = (num_sms > 0 && num_sms < sms) ? num_sms : sms;
         return out_dtype == PTB_BF16 ? launch_wgrad_pair<__nv_bfloat16>(g, grid, (cudaStream_t) stream)
                                      : launch_wgrad_pair<__half>(g, grid, (cudaStream_t) stream);
     }
-    return launch_gemm(g, mode, out_dtype, num_sms, (cudaStream_t) stream);
+    return launch_gemm(g, mode, out_dtype, grid, (cudaStream_t) stream);
 }
 
 #pragma GCC visibility pop
