@@ -87,6 +87,13 @@ int ptb_quant_fp8_tensorwise_with_scale(const void *x, int x_dtype, int64_t n, c
 int ptb_quant_fp8_rowwise(const void *x, int x_dtype, int64_t B, int64_t M, int64_t N, void *q,
                           int q_dtype, float *scale_inv, void *workspace, ptb_stream_t stream);
 
+/* The other-direction copy of a rowwise operand: q_rows is FP8 [B, M, N] with one inverse scale per row
+ * (row_scale [B, M]); the values hp_dtype(float(q_rows) * row_scale) are quantised to the same FP8 type with one scale per
+ * (b, n) over the M axis (scale_inv [B,1,N]).  Same result as ptb_dequant_fp8_rowwise to hp_dtype followed by
+ * ptb_quant_fp8_rowwise, without the tensor between them.  workspace: B*N floats, cleared by the call. */
+int ptb_requant_fp8_rowwise(const void *q_rows, int fp8_dtype, const float *row_scale, int hp_dtype, int64_t B, int64_t M,
+                            int64_t N, void *q, float *scale_inv, void *workspace, ptb_stream_t stream);
+
 /* Rowwise quantize that allocates nothing and needs no workspace argument.
  * For hosts that are not allowed to obtain device memory on the library's behalf: an inference or
  * training runtime that hands a plugin only its input and output buffers and owns every other byte

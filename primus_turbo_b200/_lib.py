@@ -38,6 +38,7 @@ _PROTOS = {
     "ptb_quant_fp8_tensorwise_with_scale": [_P, _I, _L, _P, _P, _I, _P, _P],
     "ptb_quant_fp8_rowwise": [_P, _I, _L, _L, _L, _P, _I, _P, _P, _P],
     "ptb_quant_fp8_rowwise_noalloc": [_P, _I, _L, _L, _L, _P, _I, _P, _P],
+    "ptb_requant_fp8_rowwise": [_P, _I, _P, _I, _L, _L, _L, _P, _P, _P, _P],
     "ptb_quant_fp8_block1d": [_P, _I, _L, _L, _I, _P, _I, _P, _P],
     "ptb_quant_fp8_block1d_dual": [_P, _I, _L, _L, _P, _P, _P, _P, _I, _P],
     "ptb_quant_fp8_block2d": [_P, _I, _L, _L, _L, _P, _I, _P, _P],
@@ -110,7 +111,7 @@ def check(rc: int, what: str) -> None:
 
 
 # kernels enqueued by one successful call of each entry point (memset nodes not counted)
-KERNELS_PER_CALL = {"ptb_quant_fp8_tensorwise": 2, "ptb_quant_fp8_rowwise": 2, "ptb_quant_fp8_rowwise_noalloc": 2,
+KERNELS_PER_CALL = {"ptb_quant_fp8_tensorwise": 2, "ptb_quant_fp8_rowwise": 2, "ptb_quant_fp8_rowwise_noalloc": 2, "ptb_requant_fp8_rowwise": 2,
                     "ptb_quant_fp8_segment_row_col": 2, "ptb_quant_mxfp8_grouped": 2, "ptb_moe_row_id_map": 3, "ptb_swiglu_quant_fp8_segment_row_col": 2,
                     "ptb_gemm_status": 0, "ptb_copy_segments_status": 0, "ptb_enable_peer_access": 0}
 # PTB_DEBUG_STATUS=1: after every GEMM call, wait for the device and raise if a bounded wait inside the

@@ -168,6 +168,28 @@ template <> struct RowFrag<float> {
     }
 };
 
+// Largest magnitude of one 16-byte vector, folded into a running maximum.  16-bit types stay packed (two values an
+// instruction, exact: a maximum rounds nothing, and like fmaxf it passes over a NaN).
+template <typename T> struct AbsMax {
+    typename Packed2<T>::type m;
+    __device__ __forceinline__ AbsMax() : m(Packed2<T>::zero()) {}
+    __device__ __forceinline__ void add(const uint4 &raw) {
+        using T2    = typename Packed2<T>::type;
+        const T2 *e = reinterpret_cast<const T2 *>(&raw);
+        m = __hmax2(m, __hmax2(__hmax2(__habs2(e[0]), __habs2(e[1])), __hmax2(__habs2(e[2]), __habs2(e[3]))));
+    }
+    __device__ __forceinline__ float value() const { return fmaxf(to_f32(m.x), to_f32(m.y)); }
+};
+template <> struct AbsMax<float> {
+    float m = 0.0f;
+    __device__ __forceinline__ void add(const uint4 &raw) {
+        const float *e = reinterpret_cast<const float *>(&raw);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) m = fmaxf(m, fabsf(e[j]));
+    }
+    __device__ __forceinline__ float value() const { return m; }
+};
+
 // var_k_lens[g] = ceil(len_g / 128) * 128 and its exclusive prefix var_k_offs[G+1] (one CTA).  With a
 // block table, also: for every 128-row block of the padded layout, the first source row it holds and
 // the end of its group's source rows -- so the tile kernel finds its rows with one load instead of
@@ -689,21 +711,30 @@ int launch_block_quant(BlockQuantArgs a, int x_dtype, int q_dtype, cudaStream_t 
 }
 
 // ---- tensorwise -------------------------------------------------------------------------------
+// Bound by HBM reads.  Several independent 16-byte loads per thread: with one, 2048 threads keep 32 KiB per SM in
+// flight, less than the latency times the rate.  16384 x 7168 bf16: 51 us with one, 47 with four (with eight 51 again).
+constexpr int kInFlight = 4;
+
 template <typename T> __global__ void __launch_bounds__(512) amax_kernel(const T *__restrict__ x, int64_t n,
                                                                           unsigned *amax_bits) {
     __shared__ float s_red[16];
     constexpr int V = 16 / sizeof(T); // elements per 16-byte load
-    float m = 0.0f;
     const int64_t nvec = ((reinterpret_cast<uintptr_t>(x) & 15u) == 0) ? n / V : 0;
     const int64_t gtid = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t gsz  = (int64_t) gridDim.x * blockDim.x;
-    for (int64_t i = gtid; i < nvec; i += gsz) {
-        uint4 raw = reinterpret_cast<const uint4 *>(x)[i];
-        const T *e = reinterpret_cast<const T *>(&raw);
+    const uint4 *xv    = reinterpret_cast<const uint4 *>(x);
+    AbsMax<T> am;
+    int64_t i = gtid;
+    for (; i + (kInFlight - 1) * gsz < nvec; i += kInFlight * gsz) {
+        uint4 raw[kInFlight];
 #pragma unroll
-        for (int j = 0; j < V; ++j) m = fmaxf(m, fabsf(to_f32(e[j])));
+        for (int u = 0; u < kInFlight; ++u) raw[u] = xv[i + u * gsz];
+#pragma unroll
+        for (int u = 0; u < kInFlight; ++u) am.add(raw[u]);
     }
-    for (int64_t i = nvec * V + gtid; i < n; i += gsz) m = fmaxf(m, fabsf(to_f32(x[i])));
+    for (; i < nvec; i += gsz) am.add(xv[i]);
+    float m = am.value();
+    for (int64_t j = nvec * V + gtid; j < n; j += gsz) m = fmaxf(m, fabsf(to_f32(x[j])));
     m = warp_max(m);
     if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = m;
     __syncthreads();
@@ -732,17 +763,36 @@ __global__ void __launch_bounds__(512) quant_tensorwise_kernel(const T *__restri
     const int64_t n8   = vec ? n / 8 : 0;
     const int64_t gtid = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t gsz  = (int64_t) gridDim.x * blockDim.x;
-    for (int64_t i = gtid; i < n8; i += gsz) {
+    // From the end to the start: what the maximum pass read last is still in L2 (126 MB), what it read first is not.
+    int64_t i = gtid;
+    if constexpr (sizeof(T) == 2) {
+        const uint4 *xv  = reinterpret_cast<const uint4 *>(x);
+        const float2 s2[4] = {make_float2(sc, sc), make_float2(sc, sc), make_float2(sc, sc), make_float2(sc, sc)};
+        for (; i + (kInFlight - 1) * gsz < n8; i += kInFlight * gsz) {
+            uint4 raw[kInFlight];
+#pragma unroll
+            for (int u = 0; u < kInFlight; ++u) raw[u] = __ldcs(xv + (n8 - 1 - (i + u * gsz)));
+#pragma unroll
+            for (int u = 0; u < kInFlight; ++u) scale_store8_t<FMT, T>(raw[u], s2, q + (n8 - 1 - (i + u * gsz)) * 8);
+        }
+    }
+    for (; i < n8; i += gsz) {
         float v[8];
-        load8<T>(x, i * 8, n, true, v);
+        const int64_t k = n8 - 1 - i;
+        load8<T>(x, k * 8, n, true, v);
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[j] = quant_val<FMT>(v[j], sc);
-        store8_fp8<FMT>(q, i * 8, n, true, v);
+        store8_fp8<FMT>(q, k * 8, n, true, v);
     }
-    for (int64_t i = n8 * 8 + gtid; i < n; i += gsz) q[i] = cvt_fp8<FMT>(quant_val<FMT>(to_f32(x[i]), sc));
+    for (i = n8 * 8 + gtid; i < n; i += gsz) q[i] = cvt_fp8<FMT>(quant_val<FMT>(to_f32(x[i]), sc));
 }
 
-// ---- rowwise, reduction axis contiguous: one CTA per row, two scans of the row ----------------
+// ---- rowwise, reduction axis contiguous: one CTA per row ----------------------------------------
+// A 16-bit row of at most kRowFrags * 2048 elements is read once, all loads in flight together, and stays in
+// registers between the maximum and the conversion (16384 x 8192 and two more operands of a training step: 210 us
+// with two scans, 145 so); longer rows, fp32 rows and unaligned ones are scanned twice.
+constexpr int kRowFrags = 4;
+
 template <typename T, int FMT>
 __global__ void __launch_bounds__(256) quant_rowwise_inner_kernel(const T *__restrict__ x, int64_t inner,
                                                                    uint8_t *__restrict__ q,
@@ -753,6 +803,35 @@ __global__ void __launch_bounds__(256) quant_rowwise_inner_kernel(const T *__res
     uint8_t *qr       = q + row * inner;
     const bool vec    = (inner % 8 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15u) == 0) &&
                      ((reinterpret_cast<uintptr_t>(q) & 7u) == 0);
+    if constexpr (sizeof(T) == 2) {
+        if (vec && inner <= kRowFrags * 256 * 8) { // the same for every thread of the grid
+            uint4 raw[kRowFrags];
+            AbsMax<T> am;
+#pragma unroll
+            for (int u = 0; u < kRowFrags; ++u) {
+                const int64_t c = ((int64_t) threadIdx.x + 256 * u) * 8;
+                raw[u] = c < inner ? *reinterpret_cast<const uint4 *>(xr + c) : make_uint4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int u = 0; u < kRowFrags; ++u) am.add(raw[u]);
+            float m = warp_max(am.value());
+            if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = m;
+            __syncthreads();
+            m = s_red[0];
+#pragma unroll
+            for (int k = 1; k < 8; ++k) m = fmaxf(m, s_red[k]);
+            float sc, sci;
+            scale_from_amax<FMT>(m, kEpsTensorRow, sc, sci);
+            if (threadIdx.x == 0) scale_inv[row] = sci;
+            const float2 s2[4] = {make_float2(sc, sc), make_float2(sc, sc), make_float2(sc, sc), make_float2(sc, sc)};
+#pragma unroll
+            for (int u = 0; u < kRowFrags; ++u) {
+                const int64_t c = ((int64_t) threadIdx.x + 256 * u) * 8;
+                if (c < inner) scale_store8_t<FMT, T>(raw[u], s2, qr + c);
+            }
+            return;
+        }
+    }
     float m = 0.0f;
     for (int64_t c = (int64_t) threadIdx.x * 8; c < inner; c += 256 * 8) {
         float v[8];
@@ -780,26 +859,108 @@ __global__ void __launch_bounds__(256) quant_rowwise_inner_kernel(const T *__res
 
 // ---- rowwise, reduction axis strided: x [B, M, N], reduce over M ------------------------------
 // CTA = 32 column fragments (256 columns) x 8 row lanes, over a chunk of kColChunk rows.
-constexpr int kColChunk = 128;
+//
+// SRC = 0: x holds T.  SRC = an FP8 format: x holds FP8 with one inverse scale per row, and the value quantised is what
+// dequantising would have stored, T(float(x) * row_scale): the other-direction copy of a rowwise operand is made in two
+// reads of one byte an element, where a dequantised tensor costs a write and two reads of two bytes more
+// (16384 x 8192 + 8192 x 8192 e4m3 -> e4m3: 350 us with the tensor, 181 so).  Whole vectors of 16-bit T take a
+// packed form with kColRows rows of a thread in flight.
+constexpr int kColChunk = 128, kColRows = 4;
 
-template <typename T>
-__global__ void __launch_bounds__(256) col_amax_kernel(const T *__restrict__ x, int64_t M, int64_t N,
-                                                        unsigned *__restrict__ amax_bits) {
+template <typename T, int SRC>
+__device__ __forceinline__ void load8_src(const void *__restrict__ base, int64_t row, int64_t col, int64_t N, bool vec,
+                                          const float *__restrict__ row_scale, float (&v)[8]) {
+    if constexpr (SRC == 0) {
+        load8<T>(reinterpret_cast<const T *>(base) + row * N, col, N, vec, v);
+    } else {
+        const uint8_t *r = reinterpret_cast<const uint8_t *>(base) + row * N;
+        const float s    = row_scale[row];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = (col + i < N) ? to_f32(from_f32<T>(fp8_to_f32<SRC>(r[col + i]) * s)) : 0.0f;
+    }
+}
+__device__ __forceinline__ uint32_t to_pair(float2 v, __nv_bfloat16) {
+    const __nv_bfloat162 t = __float22bfloat162_rn(v);
+    return *reinterpret_cast<const uint32_t *>(&t);
+}
+__device__ __forceinline__ uint32_t to_pair(float2 v, __half) {
+    const __half2 t = __float22half2_rn(v);
+    return *reinterpret_cast<const uint32_t *>(&t);
+}
+template <int SRC> struct SrcRaw { using type = uint2; static constexpr int kBytes = 1; };
+template <> struct SrcRaw<0> { using type = uint4; static constexpr int kBytes = 2; };
+// eight values as stored bits of a 16-bit T
+template <typename T, int SRC> __device__ __forceinline__ uint4 src_pairs(const typename SrcRaw<SRC>::type &raw, float s) {
+    if constexpr (SRC == 0) {
+        return raw;
+    } else {
+        uint4 o;
+        uint32_t *w          = reinterpret_cast<uint32_t *>(&o);
+        const uint32_t in[2] = {raw.x, raw.y};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const __nv_fp8x2_storage_t b = (__nv_fp8x2_storage_t) (in[i >> 1] >> (16 * (i & 1)));
+            const __half2_raw h          = __nv_cvt_fp8x2_to_halfraw2(b, SRC == PTB_E4M3 ? __NV_E4M3 : __NV_E5M2);
+            w[i] = to_pair(__fmul2_rn(__half22float2(*reinterpret_cast<const __half2 *>(&h)), make_float2(s, s)), T());
+        }
+        return o;
+    }
+}
+template <typename T, int SRC> __device__ __forceinline__ bool src_vec(const void *x, int64_t N) {
+    return (N % 8 == 0) && ((reinterpret_cast<uintptr_t>(x) & (SRC == 0 ? 15u : 7u)) == 0);
+}
+
+template <typename T, int SRC>
+__global__ void __launch_bounds__(256) col_amax_kernel(const void *__restrict__ x, const float *__restrict__ row_scale,
+                                                        int64_t M, int64_t N, unsigned *__restrict__ amax_bits) {
     __shared__ float s_m[8][256 + 1];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int64_t b   = blockIdx.z;
     const int64_t col = (int64_t) blockIdx.x * 256 + tx * 8;
-    const int64_t r0  = (int64_t) blockIdx.y * kColChunk;
-    const int64_t r1  = min(r0 + kColChunk, M);
-    const T *xb       = x + b * M * N;
-    const bool vec    = (N % 8 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15u) == 0);
+    const int64_t r0  = b * M + (int64_t) blockIdx.y * kColChunk; // rows are counted over the whole batch
+    const int64_t r1  = min(r0 + kColChunk, (b + 1) * M);
+    const bool vec    = src_vec<T, SRC>(x, N);
     float cm[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) cm[j] = 0.0f;
     if (col < N) {
-        for (int64_t r = r0 + ty; r < r1; r += 8) {
+        int64_t r = r0 + ty;
+        if constexpr (sizeof(T) == 2) {
+            if (vec) { // N % 8 == 0: the whole vector is inside
+                using T2  = typename Packed2<T>::type;
+                using Raw = typename SrcRaw<SRC>::type;
+                const uint8_t *src = reinterpret_cast<const uint8_t *>(x) + (r * N + col) * SrcRaw<SRC>::kBytes;
+                const int64_t step = 8 * N * SrcRaw<SRC>::kBytes;
+                T2 cm2[4];
+#pragma unroll
+                for (int w = 0; w < 4; ++w) cm2[w] = Packed2<T>::zero();
+                for (; r + 8 * (kColRows - 1) < r1; r += 8 * kColRows, src += kColRows * step) {
+                    Raw raw[kColRows];
+                    float s[kColRows];
+#pragma unroll
+                    for (int u = 0; u < kColRows; ++u) {
+                        raw[u] = *reinterpret_cast<const Raw *>(src + u * step);
+                        if constexpr (SRC != 0) s[u] = row_scale[r + 8 * u];
+                        else s[u] = 1.0f;
+                    }
+#pragma unroll
+                    for (int u = 0; u < kColRows; ++u) {
+                        const uint4 p = src_pairs<T, SRC>(raw[u], s[u]);
+                        const T2 *e   = reinterpret_cast<const T2 *>(&p);
+#pragma unroll
+                        for (int w = 0; w < 4; ++w) cm2[w] = __hmax2(cm2[w], __habs2(e[w]));
+                    }
+                }
+#pragma unroll
+                for (int w = 0; w < 4; ++w) {
+                    cm[2 * w]     = to_f32(cm2[w].x);
+                    cm[2 * w + 1] = to_f32(cm2[w].y);
+                }
+            }
+        }
+        for (; r < r1; r += 8) {
             float v[8];
-            load8<T>(xb + r * N, col, N, vec, v);
+            load8_src<T, SRC>(x, r, col, N, vec, row_scale, v);
 #pragma unroll
             for (int j = 0; j < 8; ++j) cm[j] = fmaxf(cm[j], fabsf(v[j]));
         }
@@ -816,21 +977,19 @@ __global__ void __launch_bounds__(256) col_amax_kernel(const T *__restrict__ x, 
     }
 }
 
-template <typename T, int FMT>
-__global__ void __launch_bounds__(256) quant_rowwise_outer_kernel(const T *__restrict__ x, int64_t M, int64_t N,
-                                                                   const float *__restrict__ amax,
-                                                                   uint8_t *__restrict__ q,
-                                                                   float *__restrict__ scale_inv) {
+template <typename T, int FMT, int SRC>
+__global__ void __launch_bounds__(256) quant_rowwise_outer_kernel(const void *__restrict__ x, const float *__restrict__ row_scale,
+                                                                   int64_t M, int64_t N, const float *__restrict__ amax,
+                                                                   uint8_t *__restrict__ q, float *__restrict__ scale_inv) {
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int64_t b   = blockIdx.z;
+    // the maximum pass walked the grid upwards: walked downwards, the rows it read last come from L2
+    const int64_t b   = gridDim.z - 1 - blockIdx.z;
+    const int64_t by  = gridDim.y - 1 - blockIdx.y;
     const int64_t col = (int64_t) blockIdx.x * 256 + tx * 8;
     if (col >= N) return;
-    const int64_t r0 = (int64_t) blockIdx.y * kColChunk;
-    const int64_t r1 = min(r0 + kColChunk, M);
-    const T *xb      = x + b * M * N;
-    uint8_t *qb      = q + b * M * N;
-    const bool vec   = (N % 8 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15u) == 0) &&
-                     ((reinterpret_cast<uintptr_t>(q) & 7u) == 0);
+    const int64_t r0 = b * M + by * kColChunk;
+    const int64_t r1 = min(r0 + kColChunk, (b + 1) * M);
+    const bool vec   = src_vec<T, SRC>(x, N) && ((reinterpret_cast<uintptr_t>(q) & 7u) == 0);
     float sc[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -838,15 +997,38 @@ __global__ void __launch_bounds__(256) quant_rowwise_outer_kernel(const T *__res
         sc[j]     = 0.0f;
         if (col + j < N) {
             scale_from_amax<FMT>(amax[b * N + col + j], kEpsTensorRow, sc[j], sci);
-            if (blockIdx.y == 0 && ty == 0) scale_inv[b * N + col + j] = sci;
+            if (by == 0 && ty == 0) scale_inv[b * N + col + j] = sci;
         }
     }
-    for (int64_t r = r0 + ty; r < r1; r += 8) {
+    int64_t r = r0 + ty;
+    if constexpr (sizeof(T) == 2) {
+        if (vec) {
+            using Raw = typename SrcRaw<SRC>::type;
+            const uint8_t *src = reinterpret_cast<const uint8_t *>(x) + (r * N + col) * SrcRaw<SRC>::kBytes;
+            uint8_t *dst       = q + r * N + col;
+            const int64_t step = 8 * N;
+            const float2 s2[4] = {make_float2(sc[0], sc[1]), make_float2(sc[2], sc[3]), make_float2(sc[4], sc[5]), make_float2(sc[6], sc[7])};
+            for (; r + 8 * (kColRows - 1) < r1; r += 8 * kColRows, src += kColRows * step * SrcRaw<SRC>::kBytes, dst += kColRows * step) {
+                Raw raw[kColRows];
+                float s[kColRows];
+#pragma unroll
+                for (int u = 0; u < kColRows; ++u) {
+                    raw[u] = *reinterpret_cast<const Raw *>(src + u * step * SrcRaw<SRC>::kBytes);
+                    if constexpr (SRC != 0) s[u] = row_scale[r + 8 * u];
+                    else s[u] = 1.0f;
+                }
+#pragma unroll
+                for (int u = 0; u < kColRows; ++u)
+                    scale_store8_t<FMT, T>(src_pairs<T, SRC>(raw[u], s[u]), s2, dst + u * step);
+            }
+        }
+    }
+    for (; r < r1; r += 8) {
         float v[8];
-        load8<T>(xb + r * N, col, N, vec, v);
+        load8_src<T, SRC>(x, r, col, N, vec, row_scale, v);
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[j] = quant_val<FMT>(v[j], sc[j]);
-        store8_fp8<FMT>(qb + r * N, col, N, vec, v);
+        store8_fp8<FMT>(q + r * N, col, N, vec, v);
     }
 }
 
@@ -872,39 +1054,83 @@ __global__ void __launch_bounds__(256) dequant_kernel(const uint8_t *__restrict_
     }
 }
 
-// Vector form: one thread dequantises 16 consecutive elements of a row (one 16-byte load of FP8, 32 or 64
-// bytes of output), the row / column split is done once per vector instead of once per element, and the
-// scale is either one value for the whole vector (column blocks of 16 or more) or 16 consecutive
-// values (one scale per column).  Used whenever N is a multiple of 16 and the buffers are aligned.
+// 8 consecutive FP8 values times their scales, stored as TO
+template <typename TO, int FMT>
+__device__ __forceinline__ void dequant8(const uint2 &raw, const float (&sc)[8], TO *__restrict__ dst) {
+    const uint8_t *e = reinterpret_cast<const uint8_t *>(&raw);
+    TO o[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) o[k] = from_f32<TO>(fp8_to_f32<FMT>(e[k]) * sc[k]);
+#pragma unroll
+    for (int k = 0; k < (int) sizeof(TO) / 2; ++k) reinterpret_cast<uint4 *>(dst)[k] = reinterpret_cast<const uint4 *>(o)[k];
+}
+
+// Vector form, bound by HBM: a thread takes 8 consecutive elements (one 8-byte load; for 16-bit outputs a warp's store is
+// one run of 512 bytes -- with 16 elements a thread it had gaps of 16 bytes) and has kInFlight loads in flight.  One
+// scale for everything (tensorwise) needs no coordinates at all.  Otherwise the scale is one value for the whole
+// vector (column blocks that are a multiple of 8) or, PER_COLUMN, 8 consecutive ones, and the coordinates come from 32-bit
+// divisions (the launcher checks the range; a 64-bit division is ~80 instructions, three of them cost more than
+// the rest).  16384 x 7168 e4m3 -> bf16, tensorwise: 89 us before, 58 so.
+template <typename TO, int FMT>
+__global__ void __launch_bounds__(256) dequant_one_scale_kernel(const uint8_t *__restrict__ q, int64_t nvec,
+                                                                const float *__restrict__ scale_inv, TO *__restrict__ out) {
+    const int64_t gtid = (int64_t) blockIdx.x * blockDim.x + threadIdx.x, gsz = (int64_t) gridDim.x * blockDim.x;
+    const uint2 *qv = reinterpret_cast<const uint2 *>(q);
+    const float s1  = *scale_inv;
+    const float sc[8] = {s1, s1, s1, s1, s1, s1, s1, s1};
+    int64_t i = gtid;
+    for (; i + (kInFlight - 1) * gsz < nvec; i += kInFlight * gsz) {
+        uint2 raw[kInFlight];
+#pragma unroll
+        for (int u = 0; u < kInFlight; ++u) raw[u] = qv[i + u * gsz];
+#pragma unroll
+        for (int u = 0; u < kInFlight; ++u) dequant8<TO, FMT>(raw[u], sc, out + (i + u * gsz) * 8);
+    }
+    for (; i < nvec; i += gsz) dequant8<TO, FMT>(qv[i], sc, out + i * 8);
+}
+
+struct DequantIdx32 {
+    uint32_t vec_per_row, M, bm, bn;
+    int64_t sb, sm, sn;
+};
 template <typename TO, int FMT, bool PER_COLUMN>
-__global__ void __launch_bounds__(256) dequant_vec_kernel(const uint8_t *__restrict__ q, int64_t nvec,
-                                                           const float *__restrict__ scale_inv, DequantIdx ix,
+__global__ void __launch_bounds__(256) dequant_vec_kernel(const uint8_t *__restrict__ q, uint32_t nvec,
+                                                           const float *__restrict__ scale_inv, DequantIdx32 ix,
                                                            TO *__restrict__ out) {
-    const int64_t vec_per_row = ix.N / 16;
-    for (int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += (int64_t) gridDim.x * blockDim.x) {
-        const int64_t rw = i / vec_per_row, col = (i - rw * vec_per_row) * 16;
-        const int64_t m = rw % ix.M, b = rw / ix.M;
-        const int64_t si = b * ix.sb + (m / ix.bm) * ix.sm + (col / ix.bn) * ix.sn;
-        const uint4 raw  = *reinterpret_cast<const uint4 *>(q + i * 16);
-        const uint8_t *e = reinterpret_cast<const uint8_t *>(&raw);
-        float sc[16];
-        if constexpr (PER_COLUMN) {
+    const uint32_t gsz = gridDim.x * blockDim.x;
+    constexpr int U    = PER_COLUMN ? 2 : kInFlight;
+    const uint2 *qv    = reinterpret_cast<const uint2 *>(q);
+    for (uint64_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < nvec; i0 += (uint64_t) U * gsz) {
+        uint2 raw[U];
+        float sc[U][8];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const float4 s4 = *reinterpret_cast<const float4 *>(scale_inv + si + 4 * k);
-                sc[4 * k] = s4.x; sc[4 * k + 1] = s4.y; sc[4 * k + 2] = s4.z; sc[4 * k + 3] = s4.w;
+        for (int u = 0; u < U; ++u) {
+            const uint64_t iu = i0 + (uint64_t) u * gsz;
+            if (iu >= nvec) continue;
+            const uint32_t i  = (uint32_t) iu;
+            raw[u]            = qv[i];
+            const uint32_t rw = i / ix.vec_per_row, col = (i - rw * ix.vec_per_row) * 8;
+            const uint32_t b  = rw / ix.M, m = rw - b * ix.M;
+            const int64_t si  = b * ix.sb + (int64_t) (m / ix.bm) * ix.sm + (int64_t) (col / ix.bn) * ix.sn;
+            if constexpr (PER_COLUMN) {
+                const float4 lo = *reinterpret_cast<const float4 *>(scale_inv + si);
+                const float4 hi = *reinterpret_cast<const float4 *>(scale_inv + si + 4);
+                sc[u][0] = lo.x; sc[u][1] = lo.y; sc[u][2] = lo.z; sc[u][3] = lo.w;
+                sc[u][4] = hi.x; sc[u][5] = hi.y; sc[u][6] = hi.z; sc[u][7] = hi.w;
+            } else {
+                sc[u][0] = scale_inv[si];
             }
-        } else {
-            const float s1 = scale_inv[si];
-#pragma unroll
-            for (int k = 0; k < 16; ++k) sc[k] = s1;
         }
-        TO o[16];
 #pragma unroll
-        for (int k = 0; k < 16; ++k) o[k] = from_f32<TO>(fp8_to_f32<FMT>(e[k]) * sc[k]);
-        uint4 *dst = reinterpret_cast<uint4 *>(out + i * 16);
+        for (int u = 0; u < U; ++u) {
+            const uint64_t i = i0 + (uint64_t) u * gsz;
+            if (i >= nvec) continue;
+            if constexpr (!PER_COLUMN) {
 #pragma unroll
-        for (int k = 0; k < (int) (sizeof(TO) * 16 / 16); ++k) dst[k] = reinterpret_cast<const uint4 *>(o)[k];
+                for (int k = 1; k < 8; ++k) sc[u][k] = sc[u][0];
+            }
+            dequant8<TO, FMT>(raw[u], sc[u], out + i * 8);
+        }
     }
 }
 
@@ -914,17 +1140,27 @@ int launch_dequant(const void *q, int q_dtype, int64_t n, const float *s, const 
     PTB_REQUIRE(q && s && out, PTB_ERR_ARG, "dequant: null pointer");
     PTB_REQUIRE(is_hp(out_dtype) && is_fp8(q_dtype), PTB_ERR_ARG, "dequant: bad dtype");
     const bool per_column = ix.bn == 1 && ix.sn == 1;
-    const bool one_scale  = ix.sn == 0 || (ix.bn >= 16 && ix.bn % 16 == 0);
-    if (ix.N % 16 == 0 && (per_column || one_scale) && aligned16(q) && aligned16(out) &&
+    const bool one_scale  = ix.sn == 0 || (ix.bn >= 8 && ix.bn % 8 == 0);
+    const bool buffers    = (reinterpret_cast<uintptr_t>(q) & 7u) == 0 && aligned16(out);
+    const int64_t nvec    = n / 8;
+    const int vec_blocks  = (int) imin(cdiv<int64_t>(nvec, 256 * kInFlight), 148 * 8);
+    if (n % 8 == 0 && buffers && ix.sn == 0 && ix.sm == 0 && ix.sb == 0) {
+        PTB_SWITCH_HP(out_dtype, TO, PTB_SWITCH_FP8(q_dtype, FMT,
+            (dequant_one_scale_kernel<TO, FMT><<<vec_blocks, 256, 0, st>>>((const uint8_t *) q, nvec, s, (TO *) out))));
+        PTB_LAUNCH_CHECK("dequant_one_scale_kernel");
+        return 0;
+    }
+    if (ix.N % 8 == 0 && (per_column || one_scale) && buffers && nvec < 2147483647LL && ix.N < 2147483647LL &&
         (!per_column || (aligned16(s) && ix.sb % 4 == 0 && ix.sm % 4 == 0))) {
-        const int64_t nvec = n / 16;
-        const int blocks   = (int) imin(cdiv<int64_t>(nvec, 256), 148 * 32);
+        const int64_t cap = 2147483647LL; // a block at least as long as its axis is the whole axis
+        const DequantIdx32 v{(uint32_t) (ix.N / 8), (uint32_t) imin(ix.M, cap), (uint32_t) imin(ix.bm, cap),
+                             (uint32_t) imin(ix.bn, cap), ix.sb, ix.sm, ix.sn};
         if (per_column) {
             PTB_SWITCH_HP(out_dtype, TO, PTB_SWITCH_FP8(q_dtype, FMT,
-                (dequant_vec_kernel<TO, FMT, true><<<blocks, 256, 0, st>>>((const uint8_t *) q, nvec, s, ix, (TO *) out))));
+                (dequant_vec_kernel<TO, FMT, true><<<vec_blocks, 256, 0, st>>>((const uint8_t *) q, (uint32_t) nvec, s, v, (TO *) out))));
         } else {
             PTB_SWITCH_HP(out_dtype, TO, PTB_SWITCH_FP8(q_dtype, FMT,
-                (dequant_vec_kernel<TO, FMT, false><<<blocks, 256, 0, st>>>((const uint8_t *) q, nvec, s, ix, (TO *) out))));
+                (dequant_vec_kernel<TO, FMT, false><<<vec_blocks, 256, 0, st>>>((const uint8_t *) q, (uint32_t) nvec, s, v, (TO *) out))));
         }
         PTB_LAUNCH_CHECK("dequant_vec_kernel");
         return 0;
@@ -1049,11 +1285,32 @@ int ptb_quant_fp8_rowwise(const void *x, int x_dtype, int64_t B, int64_t M, int6
     PTB_REQUIRE(B <= 65535 && cdiv<int64_t>(M, kColChunk) <= 65535, PTB_ERR_TOO_LARGE, "quant_rowwise: grid too large");
     PTB_CUDA(cudaMemsetAsync(workspace, 0, sizeof(float) * B * N, st));
     dim3 grid((unsigned) cdiv<int64_t>(N, 256), (unsigned) imax(1, cdiv<int64_t>(M, kColChunk)), (unsigned) B);
-    PTB_SWITCH_HP(x_dtype, T, (col_amax_kernel<T><<<grid, 256, 0, st>>>((const T *) x, M, N, (unsigned *) workspace)));
+    PTB_SWITCH_HP(x_dtype, T, (col_amax_kernel<T, 0><<<grid, 256, 0, st>>>(x, nullptr, M, N, (unsigned *) workspace)));
     PTB_LAUNCH_CHECK("col_amax_kernel");
     PTB_SWITCH_HP(x_dtype, T, PTB_SWITCH_FP8(q_dtype, FMT,
-        (quant_rowwise_outer_kernel<T, FMT><<<grid, 256, 0, st>>>((const T *) x, M, N, (const float *) workspace,
-                                                                   (uint8_t *) q, scale_inv))));
+        (quant_rowwise_outer_kernel<T, FMT, 0><<<grid, 256, 0, st>>>(x, nullptr, M, N, (const float *) workspace, (uint8_t *) q,
+                                                                     scale_inv))));
+    PTB_LAUNCH_CHECK("quant_rowwise_outer_kernel");
+    return 0;
+}
+
+int ptb_requant_fp8_rowwise(const void *q_rows, int fp8_dtype, const float *row_scale, int hp_dtype, int64_t B, int64_t M,
+                            int64_t N, void *q, float *scale_inv, void *workspace, ptb_stream_t stream) {
+    PTB_REQUIRE(B >= 0 && M >= 0 && N >= 0, PTB_ERR_ARG, "requant_rowwise: negative size");
+    PTB_REQUIRE(is_hp(hp_dtype) && is_fp8(fp8_dtype), PTB_ERR_ARG, "requant_rowwise: bad dtype");
+    if (B * N == 0) return 0;
+    PTB_REQUIRE(scale_inv && workspace, PTB_ERR_ARG, "requant_rowwise: null scale_inv/workspace");
+    PTB_REQUIRE(M == 0 || (q_rows && row_scale && q), PTB_ERR_ARG, "requant_rowwise: null pointer");
+    PTB_REQUIRE(B <= 65535 && cdiv<int64_t>(M, kColChunk) <= 65535, PTB_ERR_TOO_LARGE, "requant_rowwise: grid too large");
+    cudaStream_t st = (cudaStream_t) stream;
+    PTB_CUDA(cudaMemsetAsync(workspace, 0, sizeof(float) * B * N, st));
+    dim3 grid((unsigned) cdiv<int64_t>(N, 256), (unsigned) imax(1, cdiv<int64_t>(M, kColChunk)), (unsigned) B);
+    PTB_SWITCH_HP(hp_dtype, T, PTB_SWITCH_FP8(fp8_dtype, FMT,
+        (col_amax_kernel<T, FMT><<<grid, 256, 0, st>>>(q_rows, row_scale, M, N, (unsigned *) workspace))));
+    PTB_LAUNCH_CHECK("col_amax_kernel");
+    PTB_SWITCH_HP(hp_dtype, T, PTB_SWITCH_FP8(fp8_dtype, FMT,
+        (quant_rowwise_outer_kernel<T, FMT, FMT><<<grid, 256, 0, st>>>(q_rows, row_scale, M, N, (const float *) workspace,
+                                                                       (uint8_t *) q, scale_inv))));
     PTB_LAUNCH_CHECK("quant_rowwise_outer_kernel");
     return 0;
 }

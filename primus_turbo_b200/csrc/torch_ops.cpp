@@ -144,7 +144,19 @@ Tensor dequant_rowwise(const Call &c, const Tensor &q, const Tensor &s, ScalarTy
 // The other-direction companion of a rowwise copy: the dequantised values (rounded to the operand's own type)
 // quantised along `axis`.
 Quant requant_rowwise(const Call &c, const Quant &r, ScalarType hp, int64_t have_axis, int64_t axis) {
-    return quant_rowwise(c, dequant_rowwise(c, r.q, r.s, hp, have_axis), r.q.scalar_type(), axis);
+    const int64_t nd = r.q.dim(), N = r.q.size(nd - 1);
+    if (have_axis != nd - 1 || axis != nd - 2 || N == 1 || r.q.numel() == 0)
+        return quant_rowwise(c, dequant_rowwise(c, r.q, r.s, hp, have_axis), r.q.scalar_type(), axis);
+    const int64_t M = r.q.size(axis), B = r.q.numel() / (M * N);
+    auto sshape  = r.q.sizes().vec();
+    sshape[axis] = 1;
+    Quant o{c.empty(r.q.sizes(), r.q.scalar_type()), c.empty(sshape, ScalarType::Float)};
+    o.sm      = 1;
+    Tensor ws = c.empty({B * N}, ScalarType::Float);
+    check(ptb_requant_fp8_rowwise(r.q.const_data_ptr(), code_of(r.q.scalar_type()), r.scale(), code_of(hp), B, M, N,
+                                  o.q.mutable_data_ptr(), o.s.mutable_data_ptr<float>(), ws.mutable_data_ptr(), c.st),
+          "ptb_requant_fp8_rowwise", 2);
+    return o;
 }
 
 Quant quant_block_rows(const Call &c, const Tensor &x, ScalarType dt) {
