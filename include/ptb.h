@@ -260,6 +260,18 @@ int ptb_moe_row_id_map(const void *routing_map, int64_t T, int64_t E, int64_t ca
                        int32_t *row_id_map, int64_t *tokens_per_expert, int64_t *sorted_indices,
                        void *workspace, ptb_stream_t stream);
 
+/* Routing probabilities between the [T, E] table and one value per permuted row, by the row_id_map of
+ * ptb_moe_row_id_map (n = T * E entries; elem_bytes 1, 2, 4 or 8; values are moved unchanged).  _to_rows writes
+ * rows[row_id_map[i]] = probs[i] and leaves rows nobody owns alone; _to_probs writes every entry, zero where the map says -1. */
+int ptb_moe_probs_to_rows(const int32_t *row_id_map, const void *probs, int elem_bytes, int64_t n, void *rows,
+                          ptb_stream_t stream);
+int ptb_moe_rows_to_probs(const int32_t *row_id_map, const void *rows, int elem_bytes, int64_t n, void *probs,
+                          ptb_stream_t stream);
+
+/* Zeros rows [sum(counts[0..G)), n_rows) of out (row_bytes each); the sum is taken on the device. */
+int ptb_zero_rows_after(const int64_t *counts, int64_t G, int64_t n_rows, int64_t row_bytes, void *out,
+                        ptb_stream_t stream);
+
 /* out[i, :] = cast(float(in[index[i], :]) * weights[i]) over rows of H elements of type dtype (PTB_F32 /
  * PTB_F16 / PTB_BF16); an index outside [0, n_in) writes a zero row.  The backward pass of the weighted
  * un-permute (permutation.py:151-279 in the reference). */

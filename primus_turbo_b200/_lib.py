@@ -48,6 +48,9 @@ _PROTOS = {
     "ptb_dequant_fp8_block1d": [_P, _I, _L, _L, _I, _P, _P, _I, _P],
     "ptb_dequant_fp8_block2d": [_P, _I, _L, _L, _L, _P, _P, _I, _P],
     "ptb_group_offs": [_P, _L, _P, _P],
+    "ptb_moe_probs_to_rows": [_P, _P, _I, _L, _P, _P],
+    "ptb_moe_rows_to_probs": [_P, _P, _I, _L, _P, _P],
+    "ptb_zero_rows_after": [_P, _L, _L, _L, _P, _P],
     "ptb_transpose_2d_u8": [_P, _L, _L, _L, _P, _P],
     "ptb_gemm_fp8": [_P, _I, _I, _L, _P, _I, _I, _L, _P, _I, _L, _L, _L, _L, _I, _P, _L, _L, _P, _L, _L, _I, _I, _P],
     "ptb_grouped_gemm_fp8": [_P, _I, _L, _P, _I, _I, _P, _I, _L, _P, _L, _L, _L, _L, _I, _P, _L, _L, _P, _L, _L, _L,

@@ -82,51 +82,80 @@ def _unpermute(rows: torch.Tensor, row_id_map: torch.Tensor, probs: Optional[tor
     return out
 
 
+class _RowsToProbs(torch.autograd.Function):
+    """``out[t, e] = rows[row_id_map[t, e]]``, zero where the token does not go to the expert."""
+
+    @staticmethod
+    def forward(ctx, rows, row_id_map):
+        ctx.save_for_backward(row_id_map)
+        ctx.capacity = rows.shape[0]
+        rows = rows.contiguous()
+        out = torch.empty(row_id_map.shape, dtype=rows.dtype, device=rows.device)
+        with torch.cuda.device(rows.device):
+            _lib.call("ptb_moe_rows_to_probs", ptr(row_id_map), ptr(rows), rows.element_size(), row_id_map.numel(), ptr(out),
+                      stream_of(rows))
+        return out
+
+    @staticmethod
+    def backward(ctx, g):
+        return _ProbsToRows.apply(g, ctx.saved_tensors[0], ctx.capacity), None
+
+
+class _ProbsToRows(torch.autograd.Function):
+    """The other way: one value per permuted row, zero for rows nobody owns."""
+
+    @staticmethod
+    def forward(ctx, probs, row_id_map, capacity):
+        ctx.save_for_backward(row_id_map)
+        probs = probs.contiguous()
+        out = torch.zeros(capacity, dtype=probs.dtype, device=probs.device)
+        if capacity > 0:
+            with torch.cuda.device(probs.device):
+                _lib.call("ptb_moe_probs_to_rows", ptr(row_id_map), ptr(probs), probs.element_size(), row_id_map.numel(), ptr(out),
+                          stream_of(probs))
+        return out
+
+    @staticmethod
+    def backward(ctx, g):
+        return _RowsToProbs.apply(g, ctx.saved_tensors[0]), None, None
+
+
 class _Permute(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, inp, sorted_indices, row_id_map, probs, expert_of_row):
+    def forward(ctx, inp, sorted_indices, row_id_map):
         from primus_turbo_b200.pytorch.kernels.quantization_impl import gather_rows
 
-        ctx.save_for_backward(row_id_map, sorted_indices, expert_of_row)
-        ctx.T, ctx.probs_shape = inp.shape[0], None if probs is None else probs.shape
-        out = gather_rows(inp, sorted_indices)
-        permuted_probs = None
-        if probs is not None:
-            ctx.probs_dtype = probs.dtype
-            permuted_probs = probs[sorted_indices.clamp(min=0), expert_of_row] * (sorted_indices >= 0).to(probs.dtype)
-        return out, permuted_probs
+        ctx.save_for_backward(row_id_map)
+        ctx.T = inp.shape[0]
+        return gather_rows(inp, sorted_indices)
 
     @staticmethod
-    def backward(ctx, g_rows, g_probs):
-        row_id_map, sorted_indices, expert_of_row = ctx.saved_tensors
-        g_inp = _unpermute(g_rows, row_id_map, None, ctx.T) if ctx.needs_input_grad[0] else None
-        gp = None
-        if ctx.probs_shape is not None and g_probs is not None and ctx.needs_input_grad[3]:
-            gp = torch.zeros(ctx.probs_shape, dtype=g_probs.dtype, device=g_probs.device)
-            valid = (sorted_indices >= 0).to(g_probs.dtype)
-            gp.index_put_((sorted_indices.clamp(min=0), expert_of_row), g_probs * valid, accumulate=True)
-        return g_inp, None, None, gp, None
+    def backward(ctx, g_rows):
+        (row_id_map,) = ctx.saved_tensors
+        return _unpermute(g_rows, row_id_map, None, ctx.T), None, None
 
 
 class _Unpermute(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, rows, row_id_map, probs_f32, T):
-        ctx.save_for_backward(rows, row_id_map, probs_f32)
-        ctx.T = T
+    def forward(ctx, rows, row_id_map, probs_f32, T, tokens_per_expert):
+        rows = rows.contiguous()
+        ctx.save_for_backward(rows, row_id_map, probs_f32, tokens_per_expert)
         return _unpermute(rows, row_id_map, probs_f32, T)
 
     @staticmethod
     def backward(ctx, g):
-        rows, row_id_map, probs = ctx.saved_tensors
+        rows, row_id_map, probs, tokens_per_expert = ctx.saved_tensors
         g = g.contiguous()
         T, E = row_id_map.shape
-        # rows past the routed total (a caller-chosen num_out_tokens larger than it) get zero gradient
-        g_rows = torch.zeros_like(rows)
+        g_rows = torch.empty_like(rows)
         gp = torch.empty((T, E), dtype=torch.float32, device=g.device) if probs is not None else None
         with torch.cuda.device(g.device):
+            # rows past the routed total (a caller-chosen num_out_tokens larger than it) get zero gradient
+            _lib.call("ptb_zero_rows_after", ptr(tokens_per_expert), E, rows.shape[0], rows.shape[1] * rows.element_size(),
+                      ptr(g_rows), stream_of(g))
             _lib.call("ptb_unpermute_rows_bwd", ptr(g), dtype_code(g.dtype), ptr(rows), ptr(row_id_map), ptr(probs), T, E,
                       g.shape[1], ptr(g_rows), ptr(gp), stream_of(g))
-        return g_rows, None, gp, None
+        return g_rows, None, gp, None, None
 
 
 def token_permute(
@@ -162,12 +191,12 @@ def token_permute(
     else:
         capacity = int(num_out_tokens)
     row_id_map, tpe, sorted_indices = make_row_id_map(routing_map, capacity)
-    with torch.no_grad():
-        # expert of every permuted row (rows at or beyond the routed total repeat the last expert; they are
-        # only read when num_out_tokens exceeds the routed total, and then sorted_indices is unset there too)
-        bounds = torch.cumsum(tpe, 0)
-        expert_of_row = torch.searchsorted(bounds, torch.arange(capacity, device=inp.device), right=True).clamp_(max=E - 1)
-    out, permuted_probs = _Permute.apply(inp, sorted_indices, row_id_map, probs, expert_of_row)
+    out = _Permute.apply(inp, sorted_indices, row_id_map)
+    permuted_probs = None
+    if probs is not None:
+        assert probs.dim() == 2 and probs.size(0) >= T and probs.size(1) >= E and probs.device == inp.device
+        per_pair = probs if probs.shape == (T, E) else probs[:T, :E]
+        permuted_probs = _ProbsToRows.apply(per_pair, row_id_map, capacity)
     return out, permuted_probs, sorted_indices, (tpe if (return_tokens_per_expert or not fused) else None)
 
 
@@ -199,8 +228,8 @@ def token_unpermute(
     assert routing_map is not None, "routing_map must be provided (it defines where every row goes back to)"
     require_cuda(inp, routing_map)
     T = int(restore_shape[0]) if restore_shape is not None else routing_map.shape[0]
-    row_id_map, _, _ = make_row_id_map(routing_map, inp.shape[0], want_sorted=False)
+    row_id_map, tpe, _ = make_row_id_map(routing_map, inp.shape[0], want_sorted=False)
     probs = None
     if merging_probs is not None:
         probs = merging_probs.to(torch.float32).contiguous()
-    return _Unpermute.apply(inp, row_id_map, probs, T)
+    return _Unpermute.apply(inp, row_id_map, probs, T, tpe)
