@@ -13,10 +13,9 @@
 // across those four lanes, so every lane ends up holding 32 contiguous output bytes of two columns.
 #include "ptb_common.cuh"
 
-// resident CTAs per SM the quantise kernel is compiled for (measured on 16384 x 8192 bf16, both directions:
-// 2 -> 3.3 TB/s without spills, 3 -> 2.8 TB/s and 4 -> 2.6 TB/s with spills)
+// resident CTAs per SM the quantise kernel is compiled for (85 registers a thread at three)
 #ifndef PTB_MXQ_MINB
-#define PTB_MXQ_MINB 2
+#define PTB_MXQ_MINB 3
 #endif
 
 namespace ptb {
@@ -31,28 +30,20 @@ template <> struct MxFmt<PTB_E5M2> { static constexpr int mbits = 2, target_pow2
 
 // Block maximum -> biased E8M0 byte.  The maximum's mantissa is rounded to the FP8 format's width (the
 // carry may bump the exponent), the exponent of the format's largest power of two is subtracted, the
-// result is clamped to [-127, 128] and biased by 127.
-template <int FMT> __device__ __forceinline__ int mx_biased_exponent(float amax) {
-    const uint32_t bits = __float_as_uint(amax);
-    const int add       = 1 << (23 - MxFmt<FMT>::mbits - 1);
-    int e               = (int) (((bits + (uint32_t) add) >> 23) & 0x1ffu) - 127 - MxFmt<FMT>::target_pow2;
-    e                   = max(e, -127);
-    e                   = min(e, 128);
-    return e + 127;
-}
+// result is clamped to [-127, 128] and biased by 127.  A maximum is never negative and at most infinity, so the biased
+// exponent before the subtraction is at most 255 and only the lower clamp can bind.
 template <int FMT, bool ZERO_IS_ONE> __device__ __forceinline__ int mx_byte(float amax) {
     if (ZERO_IS_ONE && amax == 0.0f) return 127;
-    return mx_biased_exponent<FMT>(amax);
+    constexpr uint32_t add = 1u << (23 - MxFmt<FMT>::mbits - 1);
+    return max((int) ((__float_as_uint(amax) + add) >> 23) - MxFmt<FMT>::target_pow2, 0);
 }
 // The reference clamps a value to +-(fmax * scale), scale = (byte << 23) read as fp32, and divides by the
-// scale.  Here: multiply by the exact reciprocal 2^(127 - byte) (subnormal for bytes 254 and 255) and let the
-// saturating conversion clamp -- the same result for every finite value, because fmax * scale times the
+// scale.  Here: multiply by the exact reciprocal 2^(127 - byte) (bytes stay below 248, so it is a normal number) and let
+// the saturating conversion clamp -- the same result for every finite value, because fmax * scale times the
 // reciprocal is exactly fmax.  Byte 0 is the one exception: its scale reads as 0.0f, the clamp limit is zero
 // and every value becomes +-0, which a multiplier of zero reproduces (sign included).
 __device__ __forceinline__ float mx_inverse(int biased) {
-    const int e = 127 - biased; // 127 .. -128
-    if (biased == 0) return 0.0f;
-    return (e >= -126) ? __uint_as_float((uint32_t) (e + 127) << 23) : __uint_as_float(1u << (149 + e));
+    return biased == 0 ? 0.0f : __uint_as_float((uint32_t) (254 - biased) << 23);
 }
 
 struct MxQuantArgs {
@@ -120,157 +111,211 @@ __device__ __forceinline__ void mx_cp_async16_zfill(void *dst_smem, const void *
                  : "memory");
 }
 
-template <typename T> __device__ __forceinline__ void decode8(const uint4 &raw, float (&v)[8]) {
-    const T *e = reinterpret_cast<const T *>(&raw);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = to_f32(e[i]);
+template <typename T> struct Pair;
+template <> struct Pair<__nv_bfloat16> {
+    using type = __nv_bfloat162;
+    static __device__ __forceinline__ float2 f2(uint32_t v) { return __bfloat1622float2(*reinterpret_cast<const type *>(&v)); }
+};
+template <> struct Pair<__half> {
+    using type = __half2;
+    static __device__ __forceinline__ float2 f2(uint32_t v) { return __half22float2(*reinterpret_cast<const type *>(&v)); }
+};
+// two 16-bit values an instruction; magnitudes and maxima are exact
+template <typename T> __device__ __forceinline__ uint32_t abs2(uint32_t a) {
+    using T2 = typename Pair<T>::type;
+    const T2 r = __habs2(*reinterpret_cast<const T2 *>(&a));
+    return *reinterpret_cast<const uint32_t *>(&r);
 }
-
-template <int FMT> __device__ __forceinline__ uint32_t mx_cvt4(const float *v, float inv) {
-    float c[4];
+template <typename T> __device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) {
+    using T2 = typename Pair<T>::type;
+    const T2 r = __hmax2(*reinterpret_cast<const T2 *>(&a), *reinterpret_cast<const T2 *>(&b));
+    return *reinterpret_cast<const uint32_t *>(&r);
+}
+template <typename T> __device__ __forceinline__ uint32_t shfl_max2(uint32_t a, int lanes) {
+    return max2<T>(a, __shfl_xor_sync(0xffffffffu, a, lanes));
+}
+// four values (two packed words) times their scales -> four FP8 bytes
+template <typename T, int FMT> __device__ __forceinline__ uint32_t mx_cvt4(uint32_t lo, uint32_t hi, float2 s_lo, float2 s_hi) {
+    const float2 a = __fmul2_rn(Pair<T>::f2(lo), s_lo), b = __fmul2_rn(Pair<T>::f2(hi), s_hi);
+    return (uint32_t) cvt_fp8x2<FMT>(a.x, a.y) | ((uint32_t) cvt_fp8x2<FMT>(b.x, b.y) << 16);
+}
+__device__ __forceinline__ void store_scale_word(uint8_t *dst, uint32_t w) {
+    if ((reinterpret_cast<uintptr_t>(dst) & 3u) == 0) {
+        *reinterpret_cast<uint32_t *>(dst) = w;
+    } else {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) c[i] = __fmul_rn(v[i], inv);
-    return (uint32_t) cvt_fp8x2<FMT>(c[0], c[1]) | ((uint32_t) cvt_fp8x2<FMT>(c[2], c[3]) << 16);
+        for (int i = 0; i < 4; ++i) dst[i] = (uint8_t) (w >> (8 * i));
+    }
 }
 
 // grid: (ceil(N_pad / 128 / kMxStrip), M_pad / 128, G); 256 threads; warp w: rows 32 * (w & 3), columns 64 * (w >> 2) of a tile
 // GROUPED: blockIdx.y walks the 128-row blocks of the padded column layout; the block table says which
 // source rows it holds and where they go in the row-direction output; a block maximum of zero takes scale
 // byte 127 (1.0) instead of 0, as the reference's grouped kernel does (quantization_mxfp8.cu:1425-1450).
+//
+// Bound by HBM (4 bytes an element) once the instruction and transaction counts allow it.  Maxima stay packed in 16 bits, two
+// rows or columns a word, which halves the maximum and shuffle instructions and lets three CTAs of the SM share the
+// registers; scale bytes meet in shared memory and leave as 4-byte words at the end of the strip (a byte a store
+// was as many L2 transactions as the column copy itself); a column's 32 bytes leave in one store.  32 x 4096 x 7168
+// bf16, both directions: 976 -> 625 us; grouped activations of 8192 rows, 7168 and 4096 wide: 205 -> 96 us.
 template <typename T, int FMT, bool GROUPED>
 __global__ void __launch_bounds__(256, PTB_MXQ_MINB) mx_quant_kernel(const MxQuantArgs p) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int rl = lane >> 3, cl = lane & 7;
+    const int wr = warp & 3, wc = warp >> 2;
     const int64_t g    = GROUPED ? 0 : blockIdx.z;
-    const int64_t row0 = (int64_t) blockIdx.y * 128 + 32 * (warp & 3); // row of the (padded) column layout
+    const int64_t row0 = (int64_t) blockIdx.y * 128 + 32 * wr; // row of the (padded) column layout
     const T *x         = reinterpret_cast<const T *>(p.x) + g * p.M * p.N;
-    int64_t src0 = row0, src_end = p.M, out0 = row0; // first source row of this warp, end of valid rows, its row-output row
+    // first source row of this CTA, end of valid rows, row-output row of the first source row
+    int64_t src_blk = (int64_t) blockIdx.y * 128, src_end = p.M, out_blk = src_blk;
     if constexpr (GROUPED) {
         const int4 e = p.table[blockIdx.y];
-        src0         = (int64_t) e.x + 32 * (warp & 3);
+        src_blk      = e.x;
         src_end      = e.y;
-        out0         = (int64_t) e.z + 32 * (warp & 3);
+        out_blk      = e.z;
     }
+    const int64_t src0 = src_blk + 32 * wr + rl; // this lane's first row (then every fourth)
+    const int rows_left = (int) imin(32, imax(0, src_end - src0)); // rows src0, src0 + 4, ... that exist: 4 ps < rows_left
 
     // A CTA walks kMxStrip consecutive column tiles; the fragments of the tile after the current one are already
     // on their way (cp.async into this thread's own shared-memory slots, zero-filled outside the matrix).
     __shared__ uint4 s_frag[8][256];
+    __shared__ __align__(4) uint8_t s_rowb[128][4 * kMxStrip + 4]; // scale bytes of the strip; rows padded by a bank
+    __shared__ __align__(4) uint8_t s_colb[128 * kMxStrip][4];
     const int tiles_x = (int) (p.N_pad / 128);
     const int tx0     = (int) blockIdx.x * kMxStrip;
     const int ntiles  = min(kMxStrip, tiles_x - tx0);
     auto issue = [&](int t) {
-        const int64_t c = (int64_t) (tx0 + t) * 128 + 64 * (warp >> 2) + cl * 8;
+        const int64_t c = (int64_t) (tx0 + t) * 128 + 64 * wc + cl * 8;
+        const T *src    = x + src0 * p.N + c;
 #pragma unroll
         for (int ps = 0; ps < 8; ++ps) {
-            const int64_t r  = src0 + 4 * ps + rl;
-            const bool valid = r < src_end && c < p.N;
-            mx_cp_async16_zfill(&s_frag[ps][threadIdx.x], valid ? (const void *) (x + r * p.N + c) : (const void *) x, valid);
+            const bool valid = 4 * ps < rows_left && c < p.N;
+            mx_cp_async16_zfill(&s_frag[ps][threadIdx.x], valid ? (const void *) (src + 4 * ps * p.N) : (const void *) x, valid);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     issue(0);
     for (int t = 0; t < ntiles; ++t) {
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    uint4 raw[8];
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        uint4 raw[8];
 #pragma unroll
-    for (int ps = 0; ps < 8; ++ps) raw[ps] = s_frag[ps][threadIdx.x];
-    if (t + 1 < ntiles) issue(t + 1);
-    const int64_t col0 = (int64_t) (tx0 + t) * 128 + 64 * (warp >> 2);
-    const int64_t col  = col0 + cl * 8;
-    float rmax[8], cmax[8];
+        for (int ps = 0; ps < 8; ++ps) raw[ps] = s_frag[ps][threadIdx.x];
+        if (t + 1 < ntiles) issue(t + 1);
+        const int64_t col = (int64_t) (tx0 + t) * 128 + 64 * wc + cl * 8;
+        // cm[i]: maxima of columns 2 i, 2 i + 1 over the warp's 32 rows; rm[i]: of rows 2 i, 2 i + 1 (of this lane's eight)
+        // over the 32-column block
+        uint32_t cm[4] = {0, 0, 0, 0}, rm[4];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) cmax[j] = 0.0f;
+        for (int i = 0; i < 4; ++i) {
+            uint32_t m[2];
 #pragma unroll
-    for (int ps = 0; ps < 8; ++ps) {
-        float v[8];
-        decode8<T>(raw[ps], v);
-        float m = 0.0f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const float a = fabsf(v[j]);
-            m             = fmaxf(m, a);
-            cmax[j]       = fmaxf(cmax[j], a);
+            for (int k = 0; k < 2; ++k) {
+                const uint4 &r = raw[2 * i + k];
+                const uint32_t a0 = abs2<T>(r.x), a1 = abs2<T>(r.y), a2 = abs2<T>(r.z), a3 = abs2<T>(r.w);
+                cm[0] = max2<T>(cm[0], a0);
+                cm[1] = max2<T>(cm[1], a1);
+                cm[2] = max2<T>(cm[2], a2);
+                cm[3] = max2<T>(cm[3], a3);
+                m[k]  = max2<T>(max2<T>(a0, a1), max2<T>(a2, a3));
+            }
+            const uint32_t both = max2<T>(__byte_perm(m[0], m[1], 0x5410), __byte_perm(m[0], m[1], 0x7632));
+            rm[i]               = shfl_max2<T>(shfl_max2<T>(both, 1), 2); // the four lanes of a 32-column block
         }
-        m        = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
-        rmax[ps] = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2)); // the four lanes of a 32-column block
-    }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        cmax[j] = fmaxf(cmax[j], __shfl_xor_sync(0xffffffffu, cmax[j], 8));
-        cmax[j] = fmaxf(cmax[j], __shfl_xor_sync(0xffffffffu, cmax[j], 16)); // the four lanes that share a column
-    }
-    float tmax = 0.0f; // maximum of the 32x32 tile this lane's columns belong to
-    if (p.row_2d || p.col_2d) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) tmax = fmaxf(tmax, cmax[j]);
-        tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 1));
-        tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 2));
-    }
-
-    // ---- row direction: q_row[g][r][col .. col+7], s_row[g][r][col / 32] -----------------------------
-    if (p.q_row != nullptr) {
-        uint8_t *q       = p.q_row + g * p.M * p.N_pad;
-        uint8_t *s       = p.s_row + g * p.M * (p.N_pad / kMxBlock);
-        const int tile_b = mx_byte<FMT, GROUPED>(tmax);
-#pragma unroll
-        for (int ps = 0; ps < 8; ++ps) {
-            if (src0 + 4 * ps + rl >= src_end) continue; // only rows that exist are written
-            const int64_t r  = out0 + 4 * ps + rl;
-            const int biased = p.row_2d ? tile_b : mx_byte<FMT, GROUPED>(rmax[ps]);
-            const float inv = mx_inverse(biased);
-            float v[8];
-            decode8<T>(raw[ps], v);
-            *reinterpret_cast<uint2 *>(q + r * p.N_pad + col) = make_uint2(mx_cvt4<FMT>(v, inv), mx_cvt4<FMT>(v + 4, inv));
-            if ((cl & 3) == 0) s[r * (p.N_pad / kMxBlock) + col / kMxBlock] = (uint8_t) biased;
-        }
-    }
-
-    // ---- column direction: q_col[g][c][row0 .. row0+31] (transposed), s_col[g][c][row0 / 32] ---------
-    if (p.q_col != nullptr) {
-        uint8_t *q = p.q_col + g * p.N * p.M_pad;
-        uint8_t *s = p.s_col + g * p.N * (p.M_pad / kMxBlock);
-        const int tile_b = mx_byte<FMT, GROUPED>(tmax);
-        // two passes of four columns each keep the live state small
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            float inv[4];
+        for (int i = 0; i < 4; ++i) cm[i] = shfl_max2<T>(shfl_max2<T>(cm[i], 8), 16); // the four lanes that share a column
+        if (p.row_2d || p.col_2d) { // one maximum per 32x32 tile: every row / column of it takes that one
+            uint32_t m = max2<T>(max2<T>(cm[0], cm[1]), max2<T>(cm[2], cm[3]));
+            m          = shfl_max2<T>(shfl_max2<T>(m, 1), 2);
+            m          = max2<T>(m, __byte_perm(m, m, 0x1032));
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const int j      = 4 * h + i;
-                const int biased = p.col_2d ? tile_b : mx_byte<FMT, GROUPED>(cmax[j]);
-                inv[i] = mx_inverse(biased);
-                if (rl == 0 && col + j < p.N) s[(col + j) * (p.M_pad / kMxBlock) + row0 / kMxBlock] = (uint8_t) biased;
-            }
-            // w[ps]: this lane's row (4 ps + rl), columns 4 h .. 4 h + 3, one byte each
-            uint32_t w[8];
-#pragma unroll
-            for (int ps = 0; ps < 8; ++ps) {
-                const T *e = reinterpret_cast<const T *>(&raw[ps]) + 4 * h;
-                float c[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) c[i] = __fmul_rn(to_f32(e[i]), inv[i]);
-                w[ps] = (uint32_t) cvt_fp8x2<FMT>(c[0], c[1]) | ((uint32_t) cvt_fp8x2<FMT>(c[2], c[3]) << 16);
-            }
-            // 4x4 byte transpose across the lanes rl = 0..3 (lane bits 3 and 4): afterwards byte k of
-            // w[ps] is row 4 ps + k of column 4 h + rl
-#pragma unroll
-            for (int ps = 0; ps < 8; ++ps) {
-                uint32_t mine  = w[ps];
-                uint32_t other = __shfl_xor_sync(0xffffffffu, mine, 8);
-                mine           = (rl & 1) ? __byte_perm(mine, other, 0x3715) : __byte_perm(mine, other, 0x6240);
-                other          = __shfl_xor_sync(0xffffffffu, mine, 16);
-                mine           = (rl & 2) ? __byte_perm(mine, other, 0x3276) : __byte_perm(mine, other, 0x5410);
-                w[ps]          = mine;
-            }
-            const int64_t c = col + 4 * h + rl;
-            if (c < p.N) {
-                uint4 *dst = reinterpret_cast<uint4 *>(q + c * p.M_pad + row0);
-                dst[0]     = make_uint4(w[0], w[1], w[2], w[3]);
-                dst[1]     = make_uint4(w[4], w[5], w[6], w[7]);
+                if (p.row_2d) rm[i] = m;
+                if (p.col_2d) cm[i] = m;
             }
         }
-    }
+
+        // ---- row direction: q_row[g][r][col .. col+7], s_row[g][r][col / 32] -----------------------------
+        if (p.q_row != nullptr) {
+            uint8_t *q = p.q_row + (g * p.M + out_blk + 32 * wr + rl) * p.N_pad + col;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float2 m = Pair<T>::f2(rm[i]);
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const int ps = 2 * i + k;
+                    if (4 * ps >= rows_left) continue; // only rows that exist are written
+                    const int biased = mx_byte<FMT, GROUPED>(k ? m.y : m.x);
+                    const float inv  = mx_inverse(biased);
+                    const float2 s2  = make_float2(inv, inv);
+                    *reinterpret_cast<uint2 *>(q + 4 * ps * p.N_pad) =
+                        make_uint2(mx_cvt4<T, FMT>(raw[ps].x, raw[ps].y, s2, s2), mx_cvt4<T, FMT>(raw[ps].z, raw[ps].w, s2, s2));
+                    if ((cl & 3) == 0) s_rowb[32 * wr + 4 * ps + rl][4 * t + 2 * wc + (cl >> 2)] = (uint8_t) biased;
+                }
+            }
+        }
+
+        // ---- column direction: q_col[g][c][row0 .. row0+31] (transposed), s_col[g][c][row0 / 32] ---------
+        if (p.q_col != nullptr) {
+            uint8_t *q = p.q_col + g * p.N * p.M_pad;
+            // two passes of four columns each keep the live state small
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float2 m01 = Pair<T>::f2(cm[2 * h]), m23 = Pair<T>::f2(cm[2 * h + 1]);
+                const int b0 = mx_byte<FMT, GROUPED>(m01.x), b1 = mx_byte<FMT, GROUPED>(m01.y);
+                const int b2 = mx_byte<FMT, GROUPED>(m23.x), b3 = mx_byte<FMT, GROUPED>(m23.y);
+                const float2 s01 = make_float2(mx_inverse(b0), mx_inverse(b1)), s23 = make_float2(mx_inverse(b2), mx_inverse(b3));
+                // lane rl writes the byte of column 4 h + rl
+                s_colb[128 * t + 64 * wc + cl * 8 + 4 * h + rl][wr] = (uint8_t) (rl < 2 ? (rl == 0 ? b0 : b1) : (rl == 2 ? b2 : b3));
+                // w[ps]: this lane's row (4 ps + rl), columns 4 h .. 4 h + 3, one byte each
+                uint32_t w[8];
+#pragma unroll
+                for (int ps = 0; ps < 8; ++ps)
+                    w[ps] = h == 0 ? mx_cvt4<T, FMT>(raw[ps].x, raw[ps].y, s01, s23) : mx_cvt4<T, FMT>(raw[ps].z, raw[ps].w, s01, s23);
+                // 4x4 byte transpose across the lanes rl = 0..3 (lane bits 3 and 4): afterwards byte k of
+                // w[ps] is row 4 ps + k of column 4 h + rl
+#pragma unroll
+                for (int ps = 0; ps < 8; ++ps) {
+                    uint32_t mine  = w[ps];
+                    uint32_t other = __shfl_xor_sync(0xffffffffu, mine, 8);
+                    mine           = __byte_perm(mine, other, (rl & 1) ? 0x3715 : 0x6240);
+                    other          = __shfl_xor_sync(0xffffffffu, mine, 16);
+                    mine           = __byte_perm(mine, other, (rl & 2) ? 0x3276 : 0x5410);
+                    w[ps]          = mine;
+                }
+                const int64_t c = col + 4 * h + rl;
+                if (c < p.N) {
+                    uint8_t *dst = q + c * p.M_pad + row0; // row0 and M_pad are multiples of 32
+                    if ((reinterpret_cast<uintptr_t>(p.q_col) & 31u) == 0) {
+                        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(w[0]), "r"(w[1]),
+                                     "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                                     : "memory");
+                    } else {
+                        reinterpret_cast<uint4 *>(dst)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+                        reinterpret_cast<uint4 *>(dst)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+                    }
+                }
+            }
+        }
     } // column tiles of the strip
+
+    // ---- scale bytes of the strip: four columns' blocks, or four row blocks, per word -----------------------
+    __syncthreads();
+    if (p.q_row != nullptr) {
+        const int64_t pitch = p.N_pad / kMxBlock;
+        uint8_t *s          = p.s_row + (g * p.M + out_blk) * pitch + (int64_t) tx0 * 4;
+        for (int i = threadIdx.x; i < 128 * kMxStrip; i += 256) {
+            const int r = i / kMxStrip, t = i % kMxStrip;
+            if (t < ntiles && src_blk + r < src_end)
+                store_scale_word(s + r * pitch + 4 * t, *reinterpret_cast<const uint32_t *>(&s_rowb[r][4 * t]));
+        }
+    }
+    if (p.q_col != nullptr) {
+        const int64_t pitch = p.M_pad / kMxBlock;
+        uint8_t *s          = p.s_col + (g * p.N + (int64_t) tx0 * 128) * pitch + (int64_t) blockIdx.y * 4;
+        for (int i = threadIdx.x; i < 128 * ntiles; i += 256)
+            if ((int64_t) tx0 * 128 + i < p.N) store_scale_word(s + i * pitch, *reinterpret_cast<const uint32_t *>(s_colb[i]));
+    }
 }
 
 // out[r][c] = cast(float(q[r][c]) * (scale byte << 23 read as fp32)); TRANSPOSE writes out[c][r] instead
