@@ -1270,6 +1270,7 @@ int scale_mode_of(int granularity, int b_block_2d, int *mode) {
 } // namespace
 } // namespace ptb
 
+#include "ptb_gemm_skinny.cuh"
 #include "ptb_gemm_wgrad.cuh"
 
 // Build-time switch for A/B measurements of the two wgrad kernels (1: paired-tile kernel where it applies).
@@ -1317,6 +1318,13 @@ int ptb_gemm_fp8(const void *a, int a_dtype, int trans_a, int64_t lda, const voi
     int grid = 0;
     rc       = persistent_grid(num_sms, &grid);
     if (rc) return rc;
+    g.kind = kKindDense;
+    g.M = (int) M; g.N = (int) N; g.K = (int) K; g.G = 1;
+    g.c = c; g.ldc = ldc; g.c_group_stride = 0;
+    g.a_scale = a_scale; g.as_m = a_scale_stride_m; g.as_k = a_scale_stride_k;
+    g.b_scale = b_scale; g.bs_g = 0; g.bs_n = b_scale_stride_n; g.bs_k = b_scale_stride_k;
+    if (const int tn = skinny_rows(mode, M, 0, !trans_a && trans_b))
+        return launch_skinny(g, mode, tn, a, a_dtype, lda, b, b_dtype, ldb, 1, c_dtype, grid, (cudaStream_t) stream);
     const int ctas = dense_ctas(mode, M, N, grid);
     set_tile(g, ctas);
     // A: [M,K] K-major, or [K,M] (trans_a) MN-major
@@ -1327,15 +1335,11 @@ int ptb_gemm_fp8(const void *a, int a_dtype, int trans_a, int64_t lda, const voi
     if (trans_b) rc = make_map(&g.tm_b, b, (uint64_t) K, (uint64_t) N, 1, (uint64_t) ldb, (uint64_t) ldb * N, BN / ctas);
     else         rc = make_map(&g.tm_b, b, (uint64_t) N, (uint64_t) K, 1, (uint64_t) ldb, (uint64_t) ldb * K, BK);
     if (rc) return rc;
-    g.kind = kKindDense; g.a_mn = trans_a ? 1 : 0; g.b_mn = trans_b ? 0 : 1;
+    g.a_mn = trans_a ? 1 : 0; g.b_mn = trans_b ? 0 : 1;
     g.idesc = make_idesc(a_dtype, b_dtype, g.a_mn, g.b_mn, BN, ctas);
-    g.M = (int) M; g.N = (int) N; g.K = (int) K; g.G = 1;
     g.tiles_n = (int) cdiv<int64_t>(N, BN);
-    g.c = c; g.ldc = ldc; g.c_group_stride = 0;
     rc = make_c_map(&g.tm_c, &g.use_tma_store, c, c_dtype, (uint64_t) N, (uint64_t) M, 1, (uint64_t) ldc, 0);
     if (rc) return rc;
-    g.a_scale = a_scale; g.as_m = a_scale_stride_m; g.as_k = a_scale_stride_k;
-    g.b_scale = b_scale; g.bs_g = 0; g.bs_n = b_scale_stride_n; g.bs_k = b_scale_stride_k;
     return launch_gemm(g, mode, c_dtype, grid, (cudaStream_t) stream);
 }
 
@@ -1473,6 +1477,14 @@ int ptb_grouped_gemm_fp8(const void *a, int a_dtype, int64_t lda, const void *b,
     int grid = 0;
     rc       = persistent_grid(num_sms, &grid);
     if (rc) return rc;
+    g.kind = kKindGroupedRows;
+    g.M = (int) M_total; g.N = (int) N; g.K = (int) K; g.G = (int) G;
+    g.group_offs = group_offs;
+    g.c = out; g.ldc = ldc; g.c_group_stride = 0;
+    g.a_scale = a_scale; g.as_m = a_scale_stride_m; g.as_k = a_scale_stride_k;
+    g.b_scale = b_scale; g.bs_g = b_scale_stride_g; g.bs_n = b_scale_stride_n; g.bs_k = b_scale_stride_k;
+    if (const int tn = skinny_rows(mode, M_total, G, trans_b != 0))
+        return launch_skinny(g, mode, tn, a, a_dtype, lda, b, b_dtype, K, (uint64_t) G, out_dtype, grid, (cudaStream_t) stream);
     const int ctas = grouped_ctas(mode, M_total, G, grid);
     set_tile(g, ctas);
     rc = make_map(&g.tm_a, a, (uint64_t) K, (uint64_t) M_total, 1, (uint64_t) lda, (uint64_t) lda * M_total, BM);
@@ -1480,16 +1492,11 @@ int ptb_grouped_gemm_fp8(const void *a, int a_dtype, int64_t lda, const void *b,
     if (trans_b) rc = make_map(&g.tm_b, b, (uint64_t) K, (uint64_t) N, (uint64_t) G, (uint64_t) K, (uint64_t) K * N, BN / ctas);
     else         rc = make_map(&g.tm_b, b, (uint64_t) N, (uint64_t) K, (uint64_t) G, (uint64_t) N, (uint64_t) K * N, BK);
     if (rc) return rc;
-    g.kind = kKindGroupedRows; g.a_mn = 0; g.b_mn = trans_b ? 0 : 1;
+    g.a_mn = 0; g.b_mn = trans_b ? 0 : 1;
     g.idesc = make_idesc(a_dtype, b_dtype, g.a_mn, g.b_mn, BN, ctas);
-    g.M = (int) M_total; g.N = (int) N; g.K = (int) K; g.G = (int) G;
     g.tiles_n = (int) cdiv<int64_t>(N, BN);
-    g.group_offs = group_offs;
-    g.c = out; g.ldc = ldc; g.c_group_stride = 0;
     rc = make_c_map(&g.tm_c, &g.use_tma_store, out, out_dtype, (uint64_t) N, (uint64_t) M_total, 1, (uint64_t) ldc, 0);
     if (rc) return rc;
-    g.a_scale = a_scale; g.as_m = a_scale_stride_m; g.as_k = a_scale_stride_k;
-    g.b_scale = b_scale; g.bs_g = b_scale_stride_g; g.bs_n = b_scale_stride_n; g.bs_k = b_scale_stride_k;
     return launch_gemm(g, mode, out_dtype, grid, (cudaStream_t) stream);
 }
 
