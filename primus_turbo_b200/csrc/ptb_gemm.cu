@@ -508,6 +508,20 @@ __global__ void __launch_bounds__(Geo<BN, DEEP, CTAS>::kThreads, 1) fp8_gemm_ker
         ctl->sched_q   = (int) (gridDim.x / CTAS) / args.tiles_n;
         ctl->sched_rem = (int) (gridDim.x / CTAS) % args.tiles_n;
     }
+    if (warp == 2) {
+        if constexpr (CTAS == 2) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+                             smem_u32(&ctl->tmem_base))
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+                             smem_u32(&ctl->tmem_base))
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
+    }
+    grid_dep_begin(); // everything above touches no global memory
     if (args.kind != kKindDense) {
         for (int g = threadIdx.x; g <= args.G; g += kThreads) ctl->group_offs[g] = (int) args.group_offs[g];
     }
@@ -536,19 +550,6 @@ __global__ void __launch_bounds__(Geo<BN, DEEP, CTAS>::kThreads, 1) fp8_gemm_ker
     } else if (threadIdx.x == 0) {
         const int tiles_m = (args.M + CTAS * BM - 1) / (CTAS * BM);
         ctl->total_tiles  = (args.kind == kKindDense ? 1 : args.G) * tiles_m * args.tiles_n;
-    }
-    if (warp == 2) {
-        if constexpr (CTAS == 2) {
-            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
-                             smem_u32(&ctl->tmem_base))
-                         : "memory");
-            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-        } else {
-            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
-                             smem_u32(&ctl->tmem_base))
-                         : "memory");
-            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-        }
     }
     tc_fence_before();
     __syncthreads();
@@ -779,13 +780,13 @@ __global__ void __launch_bounds__(Geo<BN, DEEP, CTAS>::kThreads, 1) fp8_gemm_ker
                             const uint8_t *src = (i < 4 ? args.a_sf + (int64_t) row[i] * args.a_sf_ld
                                                         : args.b_sf + (b_row0 + row[i]) * args.b_sf_ld) + k_byte0 + 4 * kb0;
                             if (vec_t && kb0 + 4 <= t.num_kb) {
-                                w[i] = __ldg(reinterpret_cast<const uint4 *>(src));
+                                w[i] = *reinterpret_cast<const uint4 *>(src);
                             } else {
                                 const uint32_t *s32 = reinterpret_cast<const uint32_t *>(src);
-                                w[i].x = __ldg(s32);
-                                w[i].y = kb0 + 1 < t.num_kb ? __ldg(s32 + 1) : 0u;
-                                w[i].z = kb0 + 2 < t.num_kb ? __ldg(s32 + 2) : 0u;
-                                w[i].w = kb0 + 3 < t.num_kb ? __ldg(s32 + 3) : 0u;
+                                w[i].x = s32[0];
+                                w[i].y = kb0 + 1 < t.num_kb ? s32[1] : 0u;
+                                w[i].z = kb0 + 2 < t.num_kb ? s32[2] : 0u;
+                                w[i].w = kb0 + 3 < t.num_kb ? s32[3] : 0u;
                             }
                         }
                         loaded_kb = kb0;
@@ -1175,18 +1176,7 @@ template <int SCALE, typename OutT, int BN, int DEEP, int CTAS> int launch_bn(co
         PTB_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kSmemBytes));
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    if constexpr (CTAS == 2) {
-        cudaLaunchConfig_t cfg{};
-        cudaLaunchAttribute attr{};
-        attr.id               = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = 2;
-        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-        cfg.gridDim = dim3((unsigned) (grid & ~1)); cfg.blockDim = dim3(Geo<BN, DEEP, CTAS>::kThreads);
-        cfg.dynamicSmemBytes = kSmemBytes; cfg.stream = st; cfg.attrs = &attr; cfg.numAttrs = 1;
-        PTB_CUDA(cudaLaunchKernelEx(&cfg, kfn, args));
-    } else {
-        kfn<<<grid, Geo<BN, DEEP, CTAS>::kThreads, kSmemBytes, st>>>(args);
-    }
+    PTB_CUDA((launch_after(kfn, dim3((unsigned) (CTAS == 2 ? grid & ~1 : grid)), Geo<BN, DEEP, CTAS>::kThreads, kSmemBytes, st, CTAS, args)));
     PTB_LAUNCH_CHECK("fp8_gemm_kernel");
     return 0;
 }

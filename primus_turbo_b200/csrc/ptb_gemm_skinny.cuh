@@ -67,6 +67,7 @@ __global__ void __launch_bounds__(SkinnyGeo<TN>::kThreads, 1) skinny_gemm_kernel
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&ctl->tmem_base)) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    grid_dep_begin(); // everything above touches no global memory
     if (args.kind == kKindGroupedRows) {
         for (int g = threadIdx.x; g <= args.G; g += G_::kThreads) ctl->group_offs[g] = (int) args.group_offs[g];
         if (warp == 3) { // cumulative row tiles per group (G <= kMaxGroups, checked on the host)
@@ -268,7 +269,7 @@ template <int SCALE, typename OutT, int TN> int launch_skinny_tn(const GemmArgs 
         PTB_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) SkinnyGeo<TN>::kSmem));
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    kfn<<<grid, SkinnyGeo<TN>::kThreads, SkinnyGeo<TN>::kSmem, st>>>(args);
+    PTB_CUDA((launch_after(kfn, dim3((unsigned) grid), SkinnyGeo<TN>::kThreads, SkinnyGeo<TN>::kSmem, st, 1, args)));
     PTB_LAUNCH_CHECK("skinny_gemm_kernel");
     return 0;
 }

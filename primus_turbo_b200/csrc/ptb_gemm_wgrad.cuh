@@ -109,12 +109,13 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_pair_kernel(const __grid_
         tma_prefetch_map(&args.tm_b);
         tma_prefetch_map(&args.tm_c);
     }
-    for (int g = threadIdx.x; g <= args.G; g += kWgThreads) ctl->group_offs[g] = (int) args.group_offs[g];
     if (warp == 2) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&ctl->tmem_base))
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    grid_dep_begin(); // everything above touches no global memory
+    for (int g = threadIdx.x; g <= args.G; g += kWgThreads) ctl->group_offs[g] = (int) args.group_offs[g];
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -320,7 +321,7 @@ template <typename OutT> int launch_wgrad_pair(const GemmArgs &args, int grid, c
         PTB_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kWgSmemBytes));
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    kfn<<<grid, kWgThreads, kWgSmemBytes, st>>>(args);
+    PTB_CUDA((launch_after(kfn, dim3((unsigned) grid), kWgThreads, kWgSmemBytes, st, 1, args)));
     PTB_LAUNCH_CHECK("wgrad_pair_kernel");
     return 0;
 }

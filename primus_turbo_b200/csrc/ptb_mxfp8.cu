@@ -60,10 +60,11 @@ struct MxQuantArgs {
 // padded to `row_align` rows in the row-direction output and to 128 rows in the column-direction output.
 // One CTA: padded lengths and offsets of both layouts and the block table of MxQuantArgs; blocks past the
 // last group get an empty entry (they are written as zeros).
-__global__ void __launch_bounds__(256) mx_group_layout_kernel(const int64_t *__restrict__ group_offs, int64_t G, int64_t row_align,
-                                                              int64_t *__restrict__ row_lens, int64_t *__restrict__ row_offs,
-                                                              int64_t *__restrict__ col_lens, int64_t *__restrict__ col_offs,
-                                                              int4 *__restrict__ table, int64_t nblocks) {
+__global__ void __launch_bounds__(256) mx_group_layout_kernel(const int64_t *group_offs, int64_t G, int64_t row_align,
+                                                              int64_t *row_lens, int64_t *row_offs,
+                                                              int64_t *col_lens, int64_t *col_offs,
+                                                              int4 *table, int64_t nblocks) {
+    grid_dep_begin();
     __shared__ int64_t s_row[256], s_col[256];
     const int tid     = threadIdx.x;
     const int64_t per = cdiv<int64_t>(G, 256);
@@ -160,6 +161,7 @@ __device__ __forceinline__ void store_scale_word(uint8_t *dst, uint32_t w) {
 // bf16, both directions: 976 -> 625 us; grouped activations of 8192 rows, 7168 and 4096 wide: 205 -> 96 us.
 template <typename T, int FMT, bool GROUPED>
 __global__ void __launch_bounds__(256, PTB_MXQ_MINB) mx_quant_kernel(const MxQuantArgs p) {
+    grid_dep_begin();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int rl = lane >> 3, cl = lane & 7;
     const int wr = warp & 3, wc = warp >> 2;
@@ -375,9 +377,9 @@ int ptb_quant_mxfp8(const void *x, int x_dtype, int64_t G, int64_t M, int64_t N,
     cudaStream_t st = (cudaStream_t) stream;
     a.table = nullptr;
     if (x_dtype == PTB_BF16) {
-        PTB_SWITCH_FP8(q_dtype, FMT, (mx_quant_kernel<__nv_bfloat16, FMT, false><<<grid, 256, 0, st>>>(a)));
+        PTB_SWITCH_FP8(q_dtype, FMT, PTB_CUDA((launch_after(mx_quant_kernel<__nv_bfloat16, FMT, false>, dim3(grid), 256, 0, st, 1, a))));
     } else {
-        PTB_SWITCH_FP8(q_dtype, FMT, (mx_quant_kernel<__half, FMT, false><<<grid, 256, 0, st>>>(a)));
+        PTB_SWITCH_FP8(q_dtype, FMT, PTB_CUDA((launch_after(mx_quant_kernel<__half, FMT, false>, dim3(grid), 256, 0, st, 1, a))));
     }
     PTB_LAUNCH_CHECK("mx_quant_kernel");
     return 0;
@@ -410,15 +412,15 @@ int ptb_quant_mxfp8_grouped(const void *x, int x_dtype, int64_t M, int64_t N, co
     const int64_t nblocks = a.M_pad / kMxPad;
     PTB_REQUIRE(nblocks <= 65535, PTB_ERR_TOO_LARGE, "grouped MXFP8 quantise: more than 65535 row blocks");
     cudaStream_t st = (cudaStream_t) stream;
-    mx_group_layout_kernel<<<1, 256, 0, st>>>(group_offs, G, row_align, row_lens_padded, row_offs_padded, col_lens_padded,
-                                              col_offs_padded, (int4 *) block_table, nblocks);
+    PTB_CUDA((launch_after(mx_group_layout_kernel, dim3(1), 256, 0, st, 1, group_offs, G, row_align, row_lens_padded, row_offs_padded, col_lens_padded,
+                                              col_offs_padded, (int4 *) block_table, nblocks)));
     PTB_LAUNCH_CHECK("mx_group_layout_kernel");
     if (N == 0) return 0;
     dim3 grid((unsigned) cdiv<int64_t>(a.N_pad / 128, kMxStrip), (unsigned) nblocks, 1);
     if (x_dtype == PTB_BF16) {
-        PTB_SWITCH_FP8(q_dtype, FMT, (mx_quant_kernel<__nv_bfloat16, FMT, true><<<grid, 256, 0, st>>>(a)));
+        PTB_SWITCH_FP8(q_dtype, FMT, PTB_CUDA((launch_after(mx_quant_kernel<__nv_bfloat16, FMT, true>, dim3(grid), 256, 0, st, 1, a))));
     } else {
-        PTB_SWITCH_FP8(q_dtype, FMT, (mx_quant_kernel<__half, FMT, true><<<grid, 256, 0, st>>>(a)));
+        PTB_SWITCH_FP8(q_dtype, FMT, PTB_CUDA((launch_after(mx_quant_kernel<__half, FMT, true>, dim3(grid), 256, 0, st, 1, a))));
     }
     PTB_LAUNCH_CHECK("mx_quant_kernel");
     return 0;

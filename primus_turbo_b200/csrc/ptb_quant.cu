@@ -194,10 +194,11 @@ template <> struct AbsMax<float> {
 // block table, also: for every 128-row block of the padded layout, the first source row it holds and
 // the end of its group's source rows -- so the tile kernel finds its rows with one load instead of
 // scanning the offsets of all groups.
-__global__ void __launch_bounds__(256) segment_offsets_kernel(const int64_t *__restrict__ group_offs, int64_t G,
-                                                               int64_t *__restrict__ var_k_lens,
-                                                               int64_t *__restrict__ var_k_offs,
-                                                               int2 *__restrict__ block_table) {
+__global__ void __launch_bounds__(256) segment_offsets_kernel(const int64_t *group_offs, int64_t G,
+                                                               int64_t *var_k_lens,
+                                                               int64_t *var_k_offs,
+                                                               int2 *block_table) {
+    grid_dep_begin();
     __shared__ int64_t s_scan[256];
     const int tid     = threadIdx.x;
     const int64_t per = cdiv<int64_t>(G, 256);
@@ -254,6 +255,7 @@ __device__ __forceinline__ void cp_async16_zfill(void *dst_smem, const void *src
 
 template <typename T, int FMT>
 __global__ void __launch_bounds__(256, 3) seg_quant_stream_kernel(const BlockQuantArgs p) {
+    grid_dep_begin();
     __shared__ uint4 s_frag[8][256];
     __shared__ float s_colmax[16][kBlk + 1];
     __shared__ float s_colscale[kBlk];
@@ -360,6 +362,7 @@ __global__ void __launch_bounds__(256, 3) seg_quant_stream_kernel(const BlockQua
 // contiguous row bands (DRAM pages are used end to end instead of 256 bytes at a time).
 template <typename T, int FMT, int MODE, bool SEGMENT, int ACT = 0>
 __global__ void __launch_bounds__(256, 3) quant_block_kernel(const BlockQuantArgs p) {
+    grid_dep_begin();
     __shared__ float s_colmax[16][kBlk + 1];
     __shared__ float s_colscale[kBlk];
     __shared__ float s_red[8];
@@ -705,7 +708,7 @@ int launch_block_quant(BlockQuantArgs a, int x_dtype, int q_dtype, cudaStream_t 
                 PTB_ERR_ALIGN, "blockwise quantise: FP8 output pointers must be 8-byte aligned");
     const unsigned grid = (unsigned) (tiles_m * tiles_n);
     PTB_SWITCH_HP(x_dtype, T, PTB_SWITCH_FP8(q_dtype, FMT,
-        (quant_block_kernel<T, FMT, MODE, SEGMENT><<<grid, 256, 0, st>>>(a))));
+        PTB_CUDA((launch_after(quant_block_kernel<T, FMT, MODE, SEGMENT>, dim3(grid), 256, 0, st, 1, a)))));
     PTB_LAUNCH_CHECK("quant_block_kernel");
     return 0;
 }
@@ -787,6 +790,58 @@ __global__ void __launch_bounds__(512) quant_tensorwise_kernel(const T *__restri
     for (i = n8 * 8 + gtid; i < n; i += gsz) q[i] = cvt_fp8<FMT>(quant_val<FMT>(to_f32(x[i]), sc));
 }
 
+// A decode-sized operand (16-bit, whole aligned vectors, at most kSmallTensor elements): one cluster of eight CTAs holds it in
+// registers, exchanges the eight maxima through distributed shared memory and converts, so the clearing of the
+// maximum, the maximum pass and the second read are gone.  Bound by latency; 32 x 4096 bf16 in a decode step of a
+// 14336-wide projection: 28.7 us a step with memset and two kernels, 19.1 us with this one and overlapped launches.  Above
+// the limit the eight SMs would be the bound.
+constexpr int kSmallCtas = 8, kSmallThreads = 512, kSmallFrags = 8;
+constexpr int64_t kSmallTensor = (int64_t) kSmallCtas * kSmallThreads * kSmallFrags * 8;
+
+template <typename T, int FMT>
+__global__ void __launch_bounds__(kSmallThreads) quant_tensorwise_small_kernel(const T *x, int n8, uint8_t *q, float *scale_inv) {
+    grid_dep_begin();
+    __shared__ float s_red[kSmallThreads / 32];
+    __shared__ float s_cta[kSmallCtas]; // every CTA's maximum, written by that CTA
+    const uint4 *xv = reinterpret_cast<const uint4 *>(x);
+    const int base  = blockIdx.x * kSmallThreads + threadIdx.x;
+    uint4 raw[kSmallFrags];
+    AbsMax<T> am;
+#pragma unroll
+    for (int u = 0; u < kSmallFrags; ++u) {
+        const int i = base + u * kSmallCtas * kSmallThreads;
+        raw[u]      = i < n8 ? xv[i] : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int u = 0; u < kSmallFrags; ++u) am.add(raw[u]);
+    float m = warp_max(am.value());
+    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = m;
+    __syncthreads();
+    // a peer's shared memory may be written only once that CTA runs
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+    if (threadIdx.x < 32) {
+        m = warp_max(threadIdx.x < kSmallThreads / 32 ? s_red[threadIdx.x] : 0.0f);
+        if (threadIdx.x < kSmallCtas) {
+            uint32_t mine = (uint32_t) __cvta_generic_to_shared(&s_cta[blockIdx.x]), theirs;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(theirs) : "r"(mine), "r"(threadIdx.x));
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(theirs), "f"(m) : "memory");
+        }
+    }
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+    m = s_cta[0];
+#pragma unroll
+    for (int k = 1; k < kSmallCtas; ++k) m = fmaxf(m, s_cta[k]);
+    float sc, sci;
+    scale_from_amax<FMT>(m, kEpsTensorRow, sc, sci);
+    if (base == 0) *scale_inv = sci;
+    const float2 s2[4] = {make_float2(sc, sc), make_float2(sc, sc), make_float2(sc, sc), make_float2(sc, sc)};
+#pragma unroll
+    for (int u = 0; u < kSmallFrags; ++u) {
+        const int i = base + u * kSmallCtas * kSmallThreads;
+        if (i < n8) scale_store8_t<FMT, T>(raw[u], s2, q + (int64_t) i * 8);
+    }
+}
+
 // ---- rowwise, reduction axis contiguous: one CTA per row ----------------------------------------
 // A 16-bit row of at most kRowFrags * 2048 elements is read once, all loads in flight together, and stays in
 // registers between the maximum and the conversion (16384 x 8192 and two more operands of a training step: 210 us
@@ -794,9 +849,10 @@ __global__ void __launch_bounds__(512) quant_tensorwise_kernel(const T *__restri
 constexpr int kRowFrags = 4;
 
 template <typename T, int FMT>
-__global__ void __launch_bounds__(256) quant_rowwise_inner_kernel(const T *__restrict__ x, int64_t inner,
-                                                                   uint8_t *__restrict__ q,
-                                                                   float *__restrict__ scale_inv) {
+__global__ void __launch_bounds__(256) quant_rowwise_inner_kernel(const T *x, int64_t inner,
+                                                                   uint8_t *q,
+                                                                   float *scale_inv) {
+    grid_dep_begin();
     __shared__ float s_red[8];
     const int64_t row = blockIdx.x;
     const T *xr       = x + row * inner;
@@ -1173,8 +1229,9 @@ int launch_dequant(const void *q, int q_dtype, int64_t n, const float *s, const 
 }
 
 // ---- exclusive prefix sum of group lengths ------------------------------------------------------
-__global__ void __launch_bounds__(256) group_offs_kernel(const int64_t *__restrict__ lens, int64_t G,
-                                                          int64_t *__restrict__ offs) {
+__global__ void __launch_bounds__(256) group_offs_kernel(const int64_t *lens, int64_t G,
+                                                          int64_t *offs) {
+    grid_dep_begin();
     __shared__ int64_t s_scan[256];
     const int tid     = threadIdx.x;
     const int64_t per = cdiv<int64_t>(G, 256);
@@ -1238,6 +1295,18 @@ int ptb_quant_fp8_tensorwise(const void *x, int x_dtype, int64_t n, void *q, int
     PTB_REQUIRE(n == 0 || (x && q), PTB_ERR_ARG, "quant_tensorwise: null x/q");
     PTB_REQUIRE(is_hp(x_dtype) && is_fp8(q_dtype), PTB_ERR_ARG, "quant_tensorwise: bad dtype");
     cudaStream_t st = (cudaStream_t) stream;
+    if ((x_dtype == PTB_BF16 || x_dtype == PTB_F16) && n > 0 && n <= kSmallTensor && n % 8 == 0 && aligned16(x) &&
+        (reinterpret_cast<uintptr_t>(q) & 7u) == 0) {
+        if (x_dtype == PTB_BF16) {
+            PTB_SWITCH_FP8(q_dtype, FMT, PTB_CUDA((launch_after(quant_tensorwise_small_kernel<__nv_bfloat16, FMT>, dim3(kSmallCtas), kSmallThreads, 0, st,
+                                                                kSmallCtas, (const __nv_bfloat16 *) x, (int) (n / 8), (uint8_t *) q, scale_inv))));
+        } else {
+            PTB_SWITCH_FP8(q_dtype, FMT, PTB_CUDA((launch_after(quant_tensorwise_small_kernel<__half, FMT>, dim3(kSmallCtas), kSmallThreads, 0, st,
+                                                                kSmallCtas, (const __half *) x, (int) (n / 8), (uint8_t *) q, scale_inv))));
+        }
+        PTB_LAUNCH_CHECK("quant_tensorwise_small_kernel");
+        return 0;
+    }
     PTB_CUDA(cudaMemsetAsync(workspace, 0, sizeof(unsigned), st));
     const int blocks = (int) imax(1, imin(cdiv<int64_t>(n, 512 * 8), 148 * 4));
     if (n > 0) {
@@ -1276,8 +1345,8 @@ int ptb_quant_fp8_rowwise(const void *x, int x_dtype, int64_t B, int64_t M, int6
     if (N == 1) {
         PTB_REQUIRE(B <= 2147483647LL, PTB_ERR_TOO_LARGE, "quant_rowwise: too many rows");
         PTB_SWITCH_HP(x_dtype, T, PTB_SWITCH_FP8(q_dtype, FMT,
-            (quant_rowwise_inner_kernel<T, FMT><<<(unsigned) B, 256, 0, st>>>((const T *) x, M, (uint8_t *) q,
-                                                                               scale_inv))));
+            PTB_CUDA((launch_after(quant_rowwise_inner_kernel<T, FMT>, dim3((unsigned) B), 256, 0, st, 1, (const T *) x, M, (uint8_t *) q,
+                                                                               scale_inv)))));
         PTB_LAUNCH_CHECK("quant_rowwise_inner_kernel");
         return 0;
     }
@@ -1421,8 +1490,8 @@ int ptb_quant_fp8_segment_row_col(const void *x, int x_dtype, int64_t M, int64_t
     PTB_REQUIRE(block_table == nullptr || M < 2147483647LL, PTB_ERR_TOO_LARGE,
                 "quant_segment_row_col: the block table holds 32-bit row numbers");
     a.block_table = (const int2 *) block_table;
-    segment_offsets_kernel<<<1, 256, 0, (cudaStream_t) stream>>>(group_offs, G, var_k_lens, var_k_offs,
-                                                                  (int2 *) block_table);
+    PTB_CUDA((launch_after(segment_offsets_kernel, dim3(1), 256, 0, (cudaStream_t) stream, 1, group_offs, G, var_k_lens, var_k_offs,
+                                                                  (int2 *) block_table)));
     PTB_LAUNCH_CHECK("segment_offsets_kernel");
     if (M == 0) return 0;
     // the activation / grad-out shapes of the MoE path: 16-bit, whole column tiles, aligned rows, a block table
@@ -1434,9 +1503,9 @@ int ptb_quant_fp8_segment_row_col(const void *x, int x_dtype, int64_t M, int64_t
         const unsigned grid = (unsigned) (tiles_m * strips);
         cudaStream_t st     = (cudaStream_t) stream;
         if (x_dtype == PTB_BF16) {
-            PTB_SWITCH_FP8(q_dtype, FMT, (seg_quant_stream_kernel<__nv_bfloat16, FMT><<<grid, 256, 0, st>>>(a)));
+            PTB_SWITCH_FP8(q_dtype, FMT, PTB_CUDA((launch_after(seg_quant_stream_kernel<__nv_bfloat16, FMT>, dim3(grid), 256, 0, st, 1, a))));
         } else {
-            PTB_SWITCH_FP8(q_dtype, FMT, (seg_quant_stream_kernel<__half, FMT><<<grid, 256, 0, st>>>(a)));
+            PTB_SWITCH_FP8(q_dtype, FMT, PTB_CUDA((launch_after(seg_quant_stream_kernel<__half, FMT>, dim3(grid), 256, 0, st, 1, a))));
         }
         PTB_LAUNCH_CHECK("seg_quant_stream_kernel");
         return 0;
@@ -1464,7 +1533,7 @@ int ptb_swiglu_quant_fp8_segment_row_col(const void *x, int x_dtype, const float
     a.q_col = (uint8_t *) q_col_padded; a.s_col = s_col_padded;
     a.group_offs = group_offs; a.var_k_offs = var_k_offs; a.block_table = (const int2 *) block_table;
     cudaStream_t st = (cudaStream_t) stream;
-    segment_offsets_kernel<<<1, 256, 0, st>>>(group_offs, G, var_k_lens, var_k_offs, (int2 *) block_table);
+    PTB_CUDA((launch_after(segment_offsets_kernel, dim3(1), 256, 0, st, 1, group_offs, G, var_k_lens, var_k_offs, (int2 *) block_table)));
     PTB_LAUNCH_CHECK("segment_offsets_kernel");
     if (M == 0) return 0;
     const int64_t tiles_m = cdiv<int64_t>(M + G * kBlk, kBlk), tiles_n = cdiv<int64_t>(N, kBlk);
@@ -1473,9 +1542,9 @@ int ptb_swiglu_quant_fp8_segment_row_col(const void *x, int x_dtype, const float
                 PTB_ERR_ALIGN, "blockwise quantise: FP8 output pointers must be 8-byte aligned");
     const unsigned grid = (unsigned) (tiles_m * tiles_n);
     if (x_dtype == PTB_BF16) {
-        PTB_SWITCH_FP8(q_dtype, FMT, (quant_block_kernel<__nv_bfloat16, FMT, kModeRow | kModeCol, true, 1><<<grid, 256, 0, st>>>(a)));
+        PTB_SWITCH_FP8(q_dtype, FMT, PTB_CUDA((launch_after(quant_block_kernel<__nv_bfloat16, FMT, kModeRow | kModeCol, true, 1>, dim3(grid), 256, 0, st, 1, a))));
     } else {
-        PTB_SWITCH_FP8(q_dtype, FMT, (quant_block_kernel<__half, FMT, kModeRow | kModeCol, true, 1><<<grid, 256, 0, st>>>(a)));
+        PTB_SWITCH_FP8(q_dtype, FMT, PTB_CUDA((launch_after(quant_block_kernel<__half, FMT, kModeRow | kModeCol, true, 1>, dim3(grid), 256, 0, st, 1, a))));
     }
     PTB_LAUNCH_CHECK("quant_block_kernel");
     return 0;
@@ -1521,7 +1590,7 @@ int ptb_dequant_fp8_block2d(const void *q, int q_dtype, int64_t B, int64_t M, in
 
 int ptb_group_offs(const int64_t *group_lens, int64_t G, int64_t *group_offs, ptb_stream_t stream) {
     PTB_REQUIRE(G >= 0 && group_offs && (G == 0 || group_lens), PTB_ERR_ARG, "group_offs: bad argument");
-    group_offs_kernel<<<1, 256, 0, (cudaStream_t) stream>>>(group_lens, G, group_offs);
+    PTB_CUDA((launch_after(group_offs_kernel, dim3(1), 256, 0, (cudaStream_t) stream, 1, group_lens, G, group_offs)));
     PTB_LAUNCH_CHECK("group_offs_kernel");
     return 0;
 }

@@ -22,7 +22,7 @@ def _rows_ref(x, fp8, dim):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
-@pytest.mark.parametrize("n", [8, 4096 * 8, 4 * 592 * 512 * 8 - 8, 4 * 592 * 512 * 8 + 24, 4 * 592 * 512 * 8 + 5])
+@pytest.mark.parametrize("n", [8, 4096 * 8, 262144 - 8, 262144, 262144 + 8, 4 * 592 * 512 * 8 - 8, 4 * 592 * 512 * 8 + 24, 4 * 592 * 512 * 8 + 5])
 def test_tensorwise_pass_ends(dtype, n):
     x = torch.randn(n, device="cuda").to(dtype)
     x[-1] = 40.0  # the maximum sits in the last vector or in the element tail
