@@ -113,7 +113,8 @@ def check(rc: int, what: str) -> None:
         raise PtbError(f"{what} failed with status {rc}: {msg}")
 
 
-# kernels enqueued by one successful call of each entry point (memset nodes not counted)
+# kernels enqueued by one successful call of each entry point (memset nodes not counted; a tensorwise quantise of at most
+# 262144 elements is one, not two)
 KERNELS_PER_CALL = {"ptb_quant_fp8_tensorwise": 2, "ptb_quant_fp8_rowwise": 2, "ptb_quant_fp8_rowwise_noalloc": 2, "ptb_requant_fp8_rowwise": 2,
                     "ptb_quant_fp8_segment_row_col": 2, "ptb_quant_mxfp8_grouped": 2, "ptb_moe_row_id_map": 3, "ptb_swiglu_quant_fp8_segment_row_col": 2,
                     "ptb_gemm_status": 0, "ptb_copy_segments_status": 0, "ptb_enable_peer_access": 0}
