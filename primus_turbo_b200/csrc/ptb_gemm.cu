@@ -508,6 +508,9 @@ __global__ void __launch_bounds__(Geo<BN, DEEP, CTAS>::kThreads, 1) fp8_gemm_ker
         ctl->sched_q   = (int) (gridDim.x / CTAS) / args.tiles_n;
         ctl->sched_rem = (int) (gridDim.x / CTAS) % args.tiles_n;
     }
+    // The pair's tensor memory is allocated by both CTAs together, and barriers of one are signalled by the other: both CTAs
+    // run and have set up their barriers before either goes on.
+    if constexpr (CTAS == 2) cluster_sync();
     if (warp == 2) {
         if constexpr (CTAS == 2) {
             asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
@@ -553,7 +556,7 @@ __global__ void __launch_bounds__(Geo<BN, DEEP, CTAS>::kThreads, 1) fp8_gemm_ker
     }
     tc_fence_before();
     __syncthreads();
-    if constexpr (CTAS == 2) cluster_sync(); // the other CTA's barriers are initialised too
+    if constexpr (CTAS == 2) cluster_sync(); // the other CTA has its tensor memory too
     tc_fence_after();
     const uint32_t tmem_base = ctl->tmem_base;
 
