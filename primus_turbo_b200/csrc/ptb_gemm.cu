@@ -82,7 +82,6 @@ struct GemmArgs {
     int bn; // tile width the kernel was instantiated with
     int bm; // tile height: 128 per CTA of the tile
     int ctas; // CTAs that share a tile (1 or 2)
-    int relay; // pairs, unpadded variable-K groups: the second CTA clears its own out-of-group rows and reports its stages
     int deep; // 1: variant without output staging
     int tiles_n;
     const int64_t *group_offs;
@@ -115,11 +114,14 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
 }
-// Arrival on a barrier of the pair's other CTA.  What it hands over is tensor memory whose reads have completed
-// (tcgen05.wait::ld) or shared memory already fenced to the async proxy, so the default scope is enough; a release
-// at cluster scope waits for every outstanding access of the thread and tripled the time of the per-block modes.
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
+// Arrival on a barrier of the pair's other CTA that publishes no write: it hands tensor memory whose reads have completed
+// (tcgen05.wait::ld) back to the MMAs that overwrite it, and serves for nothing else.  A release at cluster scope waits for
+// every outstanding access of the thread and tripled the time of the per-block modes.
+__device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_bar) {
     asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ void st_zero16_cluster(uint32_t cluster_addr) {
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(cluster_addr), "r"(0) : "memory");
 }
 __device__ __forceinline__ uint32_t cluster_cta_rank() {
     uint32_t r;
@@ -312,6 +314,7 @@ struct __align__(16) SharedCtl {
     uint64_t sc_empty[kScaleSlots];
     uint64_t full[kMaxStages];
     uint64_t empty[kMaxStages];
+    uint64_t cut[kMaxStages]; // pairs, in the first CTA: both CTAs' copies of a block that reaches past its group have landed
     uint64_t tmem_full[kMaxAccBufs];
     uint64_t tmem_empty[kMaxAccBufs];
     uint32_t tmem_base;
@@ -450,14 +453,26 @@ template <> struct Pack8<float> {
 
 // The last block of an unpadded variable-K group reaches into the next group's rows (or past the last group): clear
 // those contraction rows in both MN-major operand tiles, so that whatever bytes lie there -- FP8 NaN patterns
-// included -- add nothing.  A contraction row is 128 bytes in the A tile and in each 128-column part of the B tile;
+// included -- add nothing.  Rows up to `end` only: with tensorwise and rowwise scales the MMA steps (of 32 rows) that hold
+// no valid row are not issued.  A contraction row is 128 bytes in the A tile and in each 128-column part of the B tile;
 // the swizzle only permutes bytes inside a row.  One warp.
-template <int B_PARTS> __device__ __forceinline__ void clear_tail_rows(uint8_t *a_tile, int k_tail, int lane) {
-    for (int off = k_tail * 128 + lane * 16; off < kABytes; off += 32 * 16) {
+template <int B_PARTS> __device__ __forceinline__ void clear_tail_rows(uint8_t *a_tile, int k_tail, int end, int lane) {
+    for (int off = k_tail * 128 + lane * 16; off < end * 128; off += 32 * 16) {
 #pragma unroll
         for (int p = 0; p <= B_PARTS; ++p) *reinterpret_cast<uint4 *>(a_tile + p * 16384 + off) = make_uint4(0, 0, 0, 0);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+// The same for a pair's block: the tiles of this CTA and, through `peer` (the same address in the other CTA), of the other.
+template <int B_PARTS> __device__ __forceinline__ void clear_tail_rows_pair(uint8_t *a_tile, uint32_t peer, int k_tail, int end, int lane) {
+    for (int off = k_tail * 128 + lane * 16; off < end * 128; off += 32 * 16) {
+#pragma unroll
+        for (int p = 0; p <= B_PARTS; ++p) {
+            st_zero16_cluster(peer + p * 16384 + off);
+            *reinterpret_cast<uint4 *>(a_tile + p * 16384 + off) = make_uint4(0, 0, 0, 0);
+        }
+    }
+    asm volatile("fence.proxy.async;" ::: "memory");
 }
 
 template <int SCALE, typename OutT, int BN, int DEEP, int CTAS>
@@ -477,14 +492,15 @@ __global__ void __launch_bounds__(Geo<BN, DEEP, CTAS>::kThreads, 1) fp8_gemm_ker
     const uint32_t smem_base = smem_u32(smem);
     const int rank     = CTAS == 2 ? (int) cluster_cta_rank() : 0; // this CTA's half of the tile
     const bool leader  = rank == 0;
-    const bool relayed = CTAS == 2 && args.relay;
     constexpr bool kPerBlock = (SCALE == kScaleBlock2D || SCALE == kScaleBlock1D);
+    constexpr bool kSkipSteps = SCALE == kScaleTensor || SCALE == kScaleRow; // the modes with unpadded variable-K groups
 
     // ---- set-up: barriers, tile table, tensor memory -------------------------------------------
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
-            mbar_init(smem_u32(&ctl->full[s]), relayed && leader ? 2 : 1);
+            mbar_init(smem_u32(&ctl->full[s]), 1);
             mbar_init(smem_u32(&ctl->empty[s]), 1);
+            mbar_init(smem_u32(&ctl->cut[s]), 1);
         }
         for (int b = 0; b < kAccBufs; ++b) {
             mbar_init(smem_u32(&ctl->tmem_full[b]), 1);
@@ -575,6 +591,7 @@ __global__ void __launch_bounds__(Geo<BN, DEEP, CTAS>::kThreads, 1) fp8_gemm_ker
             Schedule sched(args, ctl);
             Tile t;
             uint32_t it = 0; // ring position over the whole kernel
+            uint32_t cut = 0, cut_ph = 0; // pairs, a bit per stage: the last copies signal `cut`; the phase of that barrier
             bool ok     = true;
             while (ok && sched.get(t)) {
                 const int gb = (args.kind == kKindGroupedRows) ? t.g : 0;
@@ -586,14 +603,15 @@ __global__ void __launch_bounds__(Geo<BN, DEEP, CTAS>::kThreads, 1) fp8_gemm_ker
                     const uint32_t sa = smem_base + s * kStageBytes, sb = sa + kABytes;
                     const int k = t.k_row0 + kb * BK;
                     if constexpr (CTAS == 2) {
-                        // Both CTAs' copies complete on the first CTA's barrier, except where the second relays.  A
-                        // half of A that holds no row of the tile is not fetched: its products are never read.
+                        // Both CTAs' copies complete on the first CTA's barrier; on `cut` for a block with rows to clear, whose
+                        // `full` warp 3 completes.  A half of A that holds no row of the tile is not fetched: its
+                        // products are never read.
                         const int m0 = t.m0 + rank * BM, n0 = t.n0 + rank * (BN / 2);
-                        const bool has_a = m0 < t.m_end;
-                        uint32_t bar     = full;
-                        if (relayed) mbar_expect_tx(full, has_a ? kStageBytes : kStageBytes - kABytes);
-                        else if (leader) mbar_expect_tx(full, m0 + BM < t.m_end ? 2 * kStageBytes : 2 * kStageBytes - kABytes);
-                        if (!relayed) bar = map_to_cta(full, 0);
+                        const bool has_a = m0 < t.m_end, past = t.k_tail != 0 && kb == t.num_kb - 1;
+                        const uint32_t mine = past ? smem_u32(&ctl->cut[s]) : full, bar = map_to_cta(mine, 0);
+                        if (leader) mbar_expect_tx(mine, m0 + BM < t.m_end ? 2 * kStageBytes : 2 * kStageBytes - kABytes);
+                        cut    = past ? cut | 1u << s : cut & ~(1u << s);
+                        cut_ph ^= past ? 1u << s : 0u;
                         if (has_a) {
                             if (args.a_mn) tma_load_3d_pair(sa, &args.tm_a, bar, m0, k, 0);
                             else           tma_load_3d_pair(sa, &args.tm_a, bar, k, m0, 0);
@@ -617,33 +635,15 @@ __global__ void __launch_bounds__(Geo<BN, DEEP, CTAS>::kThreads, 1) fp8_gemm_ker
                 atomicExch(&g_gemm_status, 1);
                 // let the copies already issued land before the CTA releases its shared memory (a pair's second CTA
                 // finds its copies' barrier in the first; the pair leaves together, after the first has waited)
-                if (CTAS == 2 && !leader && !relayed) it = 0;
+                if (CTAS == 2 && !leader) it = 0;
                 const uint32_t back = it < (uint32_t) kStages ? it : (uint32_t) kStages;
                 for (uint32_t j = 1; j <= back; ++j) {
-                    const uint32_t q = it - j;
-                    mbar_wait(smem_u32(&ctl->full[q % kStages]), (q / kStages) & 1);
+                    const uint32_t q = it - j, s = q % kStages;
+                    if (CTAS == 2 && (cut >> s & 1)) mbar_wait(smem_u32(&ctl->cut[s]), (cut_ph >> s & 1) ^ 1);
+                    else mbar_wait(smem_u32(&ctl->full[s]), (q / kStages) & 1);
                 }
             }
-        } else if (warp == 1 && !leader) {
-            // ================= second CTA of a pair: reports its stages where they need work first =================
-            if (relayed) {
-                Schedule sched(args, ctl);
-                Tile t;
-                uint32_t it = 0;
-                bool ok     = true;
-                while (ok && sched.get(t)) {
-                    for (int kb = 0; kb < t.num_kb; ++kb, ++it) {
-                        const int s = it % kStages;
-                        if (!mbar_wait(smem_u32(&ctl->full[s]), (it / kStages) & 1)) { ok = false; break; }
-                        if (t.k_tail != 0 && kb == t.num_kb - 1)
-                            clear_tail_rows<G_::kBBytes / 16384>(smem + s * kStageBytes, t.k_tail, lane);
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&ctl->full[s]), 0));
-                    }
-                }
-                if (!ok && lane == 0) atomicExch(&g_gemm_status, 2);
-            }
-        } else if (warp == 1) {
+        } else if (warp == 1 && leader) {
             // ================= MMA issuer (whole warp walks the schedule, lane 0 issues) =================
             Schedule sched(args, ctl);
             Tile t;
@@ -667,7 +667,9 @@ __global__ void __launch_bounds__(Geo<BN, DEEP, CTAS>::kThreads, 1) fp8_gemm_ker
                         if (!mbar_wait(smem_u32(&ctl->sc_full[slot]), (it / kScaleSlots) & 1)) { ok = false; break; }
                     }
                     uint8_t *a_tile = smem + s * kStageBytes;
-                    if (t.k_tail != 0 && kb == t.num_kb - 1) clear_tail_rows<G_::kBBytes / 16384>(a_tile, t.k_tail, lane);
+                    const bool past = t.k_tail != 0 && kb == t.num_kb - 1; // the block reaches past its group
+                    if (CTAS == 1 && past) // (a pair's warp 3 has done it)
+                        clear_tail_rows<G_::kBBytes / 16384>(a_tile, t.k_tail, kSkipSteps ? (t.k_tail + 31) & ~31 : BK, lane);
                     __syncwarp();
                     tc_fence_after();
                     if (lane == 0) {
@@ -691,6 +693,11 @@ __global__ void __launch_bounds__(Geo<BN, DEEP, CTAS>::kThreads, 1) fp8_gemm_ker
                                             sf_tmem, sf_tmem + 4, accumulate);
                             }
                             tc_commit(smem_u32(&ctl->sc_empty[slot])); // scale slot reusable once copies and MMAs retire
+                        } else if (kSkipSteps && past) {
+#pragma unroll 1
+                            for (int j = 0; 32 * j < t.k_tail; ++j)
+                                tc_mma_f8<CTAS>(d, ad + (uint64_t) ((a_step * j) >> 4), bd + (uint64_t) ((b_step * j) >> 4), args.idesc,
+                                                (j > 0 || !new_acc) ? 1u : 0u);
                         } else {
 #pragma unroll
                             for (int j = 0; j < BK / 32; ++j) {
@@ -709,6 +716,28 @@ __global__ void __launch_bounds__(Geo<BN, DEEP, CTAS>::kThreads, 1) fp8_gemm_ker
                 }
             }
             if (!ok && lane == 0) atomicExch(&g_gemm_status, 2);
+        } else if (CTAS == 2 && warp == 3) {
+            // ================= pairs, first CTA: blocks that reach past their group =================
+            // The MMA reads both CTAs' tiles, and this warp clears both, so that the writes, the proxy fence, the stage's
+            // barrier and the MMA all lie in one CTA.  (The second CTA clearing its own half has to hand it over with a
+            // release and an acquire at cluster scope: wgrad of 64 groups of 60 rows on average, 2048 x 2048: 152 us.)
+            Schedule sched(args, ctl);
+            Tile t;
+            uint32_t it = 0, ph = 0; // ph: a bit per stage
+            while (leader && sched.get(t)) {
+                it += t.num_kb;
+                if (t.k_tail == 0) continue;
+                const int s = (it - 1) % kStages; // the tile's last block
+                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->cut[s]), ph >> s & 1))) { // the warp leaves as one
+                    if (lane == 0) atomicExch(&g_gemm_status, 2);
+                    break;
+                }
+                ph ^= 1u << s;
+                clear_tail_rows_pair<G_::kBBytes / 16384>(smem + s * kStageBytes, map_to_cta(smem_base + s * kStageBytes, 1), t.k_tail,
+                                                            (t.k_tail + 31) & ~31, lane);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&ctl->full[s]));
+            }
         } else if (warp == 3 || (SCALE == kScaleMX && warp == 2)) {
             // ================= scale loader (1-D x 1-D block scales; MX: warps 2 and 3) =================
             // Copies each contraction block's row and column scales into the ring with cp.async; the
@@ -980,7 +1009,7 @@ __global__ void __launch_bounds__(Geo<BN, DEEP, CTAS>::kThreads, 1) fp8_gemm_ker
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) { // buffer may be overwritten now
-                    if constexpr (CTAS == 2) mbar_arrive_cluster(map_to_cta(smem_u32(&ctl->tmem_empty[buf]), 0));
+                    if constexpr (CTAS == 2) mbar_arrive_cluster_relaxed(map_to_cta(smem_u32(&ctl->tmem_empty[buf]), 0));
                     else mbar_arrive(smem_u32(&ctl->tmem_empty[buf]));
                 }
                 PTB_PROMOTE(v0, 2)
@@ -1517,7 +1546,6 @@ int ptb_grouped_gemm_fp8_variable_k(const void *lhs, int lhs_dtype, int64_t ld_l
     if (rc) return rc;
     const int ctas = (mode == kScaleTensor || mode == kScaleRow) && OUT_M > BM && grid >= 2 ? 2 : 1;
     set_tile(g, ctas);
-    g.relay = mode != kScaleBlock1D; // unpadded groups: contraction rows past a group's end have to be cleared
     const uint64_t r = rows > 0 ? (uint64_t) rows : 1;
     rc = make_map(&g.tm_a, lhs, (uint64_t) OUT_M, r, 1, (uint64_t) ld_lhs, (uint64_t) ld_lhs * r, BK);
     if (rc) return rc;
