@@ -612,12 +612,27 @@ template <typename F> py::object guarded(F &&f) {
 
 bool plain_cuda(const Tensor &t) { return t.device().is_cuda() && t.layout() == at::kStrided && t.numel() > 0; }
 
+// The scales of a weight [.., rows, cols] quantised ahead of time: as the kernels read them, and as many.  Anything else -- another
+// type, a reshaped payload with the scales of its former shape -- is for the Python form, which converts or refuses.
+bool scales_fit(const Tensor &w, const Tensor &s, int gran, bool tb) {
+    if (s.device() != w.device() || s.layout() != at::kStrided) return false;
+    const int64_t nd = w.dim();
+    if (gran == kMxGranularity) {
+        if ((s.scalar_type() != ScalarType::Float8_e8m0fnu && s.scalar_type() != ScalarType::Byte) || s.dim() != nd) return false;
+        return s.sizes().slice(0, nd - 1) == w.sizes().slice(0, nd - 1) && s.size(-1) * kMxBlk == w.size(-1);
+    }
+    if (s.scalar_type() != ScalarType::Float) return false;
+    if (gran == PTB_TENSORWISE) return s.numel() == 1;
+    if (gran == PTB_ROWWISE) return s.numel() == (nd == 3 ? w.size(0) : 1) * w.size(tb ? -2 : -1);
+    return s.dim() == nd && (nd == 2 || s.size(0) == w.size(0)) && s.size(-2) == cdiv(w.size(-2), kBlk) && s.size(-1) == cdiv(w.size(-1), kBlk);
+}
+
 py::object py_gemm_fp8(const Tensor &a, const Tensor &b, const std::optional<Tensor> &b_scale, bool ta, bool tb, ScalarType out,
                        int gran, ScalarType fwd, ScalarType bwd) {
     if (!plain_cuda(a) || !plain_cuda(b) || a.device() != b.device() || a.dim() != 2 || b.dim() != 2 || !is_hp(a.scalar_type()) ||
         !is_hp(out) || a.size(ta ? 0 : 1) != b.size(tb ? 1 : 0))
         return py::none();
-    if (b_scale ? !is_fp8(b.scalar_type()) : !is_hp(b.scalar_type())) return py::none();
+    if (b_scale ? !is_fp8(b.scalar_type()) || !scales_fit(b, *b_scale, gran, tb) : !is_hp(b.scalar_type())) return py::none();
     if (gran != PTB_TENSORWISE && ta) return py::none();
     if (gran == kMxGranularity && (!tb || a.size(1) % kMxBlk || b.size(0) % kMxBlk || !is_16bit(a.scalar_type()) || !is_16bit(out) ||
                                    (!b_scale && !is_16bit(b.scalar_type()))))
@@ -644,7 +659,7 @@ py::object py_grouped_gemm_fp8(const Tensor &a, const Tensor &b, const std::opti
     if (offs && (!plain_cuda(*offs) || offs->device() != a.device() || offs->scalar_type() != ScalarType::Long ||
                  offs->numel() != b.size(0) + 1))
         return py::none();
-    if (b_scale ? !is_fp8(b.scalar_type()) : !is_hp(b.scalar_type())) return py::none();
+    if (b_scale ? !is_fp8(b.scalar_type()) || !scales_fit(b, *b_scale, gran, tb) : !is_hp(b.scalar_type())) return py::none();
     if (gran == kMxGranularity && (!tb || a.size(1) % kMxBlk || b.size(1) % kMxBlk || !is_16bit(a.scalar_type()) ||
                                    (!b_scale && !is_16bit(b.scalar_type()))))
         return py::none();

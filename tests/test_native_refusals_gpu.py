@@ -1,0 +1,62 @@
+"""GPU: calls that the native host path leaves to the Python form -- because only that refuses them, can be recorded, or
+reads what the call brings along -- and what the native path must not lose when it does take a call."""
+
+import pytest
+import torch
+
+from primus_turbo_b200.pytorch.core.low_precision import Float8QuantConfig, Format, ScaleDtype
+from primus_turbo_b200.pytorch.core.low_precision import ScalingGranularity as G
+from primus_turbo_b200.pytorch.core.quantized_tensor import QuantizedTensor, create_quantized_weight
+from primus_turbo_b200.pytorch.ops import gemm_fp8, grouped_gemm_fp8
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+E4 = torch.float8_e4m3fn
+GRANS = [G.TENSORWISE, G.ROWWISE, G.BLOCKWISE, G.MX_BLOCKWISE]
+
+
+def _config(gran, fmt=Format.E4M3):
+    block = {G.BLOCKWISE: 128, G.MX_BLOCKWISE: 32}.get(gran)
+    scale = ScaleDtype.E8M0 if gran == G.MX_BLOCKWISE else ScaleDtype.FP32
+    return Float8QuantConfig(format=fmt, granularity=gran, block_size=block, scale_dtype=scale)
+
+
+def _rand(*shape, seed=1):
+    return torch.randn(*shape, device=DEV, dtype=torch.bfloat16, generator=torch.Generator(DEV).manual_seed(seed))
+
+
+LENS = [33, 0, 67]
+
+
+def _op(grouped, gran, fmt=Format.E4M3):
+    """(op of activation and weight, activation, weight)"""
+    cfg = _config(gran, fmt)
+    if grouped:
+        lens = torch.tensor(LENS, device=DEV)
+        return lambda a, w: grouped_gemm_fp8(a, w, lens, config=cfg), _rand(100, 256), _rand(3, 384, 256, seed=2)
+    return lambda a, w: gemm_fp8(a, w, trans_b=True, config=cfg), _rand(100, 256), _rand(384, 256, seed=2)
+
+
+# ---- weights quantised ahead of time ----------------------------------------------------------------------------
+def _with_scale(q, scale):
+    return QuantizedTensor(q.qdata, scale, shape=q.shape, orig_dtype=q.dtype, dest_dtype=q.real_dtype, granularity=q.granularity,
+                           block_size=q.block_size, scaling_recipe=q.scaling_recipe, quantized_axis=-1)
+
+
+@pytest.mark.parametrize("grouped", [False, True])
+def test_a_cached_weight_whose_scales_do_not_fit_is_refused(grouped):
+    """A reshaped weight keeps its scales (``QuantizedTensor.view``): fewer than the product has columns is an error."""
+    op, _, w = _op(grouped, G.ROWWISE)
+    q, _ = create_quantized_weight(w, E4, _config(G.ROWWISE))
+    wider = q.view(*w.shape[:-2], w.shape[-2] * 2, w.shape[-1] // 2)
+    with torch.no_grad(), pytest.raises((AssertionError, RuntimeError)):
+        op(_rand(100, 128), wider)
+
+
+@pytest.mark.parametrize("grouped", [False, True])
+@pytest.mark.parametrize("gran", [G.TENSORWISE, G.ROWWISE, G.BLOCKWISE])
+def test_a_cached_weight_with_wider_scales_is_still_taken(gran, grouped):
+    op, a, w = _op(grouped, gran)
+    q, _ = create_quantized_weight(w, E4, _config(gran))
+    with torch.no_grad():
+        assert torch.equal(op(a, _with_scale(q, q.scale_inv.double())), op(a, q))
