@@ -610,6 +610,10 @@ template <typename F> py::object guarded(F &&f) {
     }
 }
 
+// The ops have no forward-mode derivative.  A tangent needs neither grad mode nor requires_grad, so a call that brings one
+// looks like inference: the Python form raises, here the tangent would be dropped.
+bool has_tangent(const Tensor &t) { return t._fw_grad(/*level=*/0).defined(); }
+
 bool plain_cuda(const Tensor &t) { return t.device().is_cuda() && t.layout() == at::kStrided && t.numel() > 0; }
 
 // The scales of a weight [.., rows, cols] quantised ahead of time: as the kernels read them, and as many.  Anything else -- another
@@ -629,6 +633,7 @@ bool scales_fit(const Tensor &w, const Tensor &s, int gran, bool tb) {
 
 py::object py_gemm_fp8(const Tensor &a, const Tensor &b, const std::optional<Tensor> &b_scale, bool ta, bool tb, ScalarType out,
                        int gran, ScalarType fwd, ScalarType bwd) {
+    if (has_tangent(a) || has_tangent(b)) return py::none();
     if (!plain_cuda(a) || !plain_cuda(b) || a.device() != b.device() || a.dim() != 2 || b.dim() != 2 || !is_hp(a.scalar_type()) ||
         !is_hp(out) || a.size(ta ? 0 : 1) != b.size(tb ? 1 : 0))
         return py::none();
@@ -652,6 +657,7 @@ py::object py_gemm_fp8(const Tensor &a, const Tensor &b, const std::optional<Ten
 py::object py_grouped_gemm_fp8(const Tensor &a, const Tensor &b, const std::optional<Tensor> &b_scale, const Tensor &lens,
                                const std::optional<Tensor> &offs, bool tb, ScalarType out, int gran, ScalarType fwd, ScalarType bwd,
                                int num_sms) {
+    if (has_tangent(a) || has_tangent(b)) return py::none();
     if (!plain_cuda(a) || !plain_cuda(b) || !plain_cuda(lens) || a.device() != b.device() || a.device() != lens.device() ||
         a.dim() != 2 || b.dim() != 3 || !is_hp(a.scalar_type()) || !is_16bit(out) || a.size(1) != b.size(tb ? 2 : 1) ||
         lens.dim() != 1 || lens.scalar_type() != ScalarType::Long || lens.size(0) != b.size(0) || !lens.is_contiguous())

@@ -3,6 +3,7 @@ reads what the call brings along -- and what the native path must not lose when 
 
 import pytest
 import torch
+import torch.autograd.forward_ad as fwAD
 
 from primus_turbo_b200.pytorch.core.low_precision import Float8QuantConfig, Format, ScaleDtype
 from primus_turbo_b200.pytorch.core.low_precision import ScalingGranularity as G
@@ -35,6 +36,25 @@ def _op(grouped, gran, fmt=Format.E4M3):
         lens = torch.tensor(LENS, device=DEV)
         return lambda a, w: grouped_gemm_fp8(a, w, lens, config=cfg), _rand(100, 256), _rand(3, 384, 256, seed=2)
     return lambda a, w: gemm_fp8(a, w, trans_b=True, config=cfg), _rand(100, 256), _rand(384, 256, seed=2)
+
+
+# ---- forward-mode differentiation -----------------------------------------------------------------------------
+@pytest.mark.parametrize("gran", GRANS)
+@pytest.mark.parametrize("grouped", [False, True])
+@pytest.mark.parametrize("dual", ["a", "w", "a, cached w"])
+@pytest.mark.parametrize("grad_mode", [True, False])
+def test_a_forward_mode_tangent_is_refused(gran, grouped, dual, grad_mode):
+    """The ops have no forward-mode derivative: a tangent raises, it is not dropped."""
+    op, a, w = _op(grouped, gran)
+    with fwAD.dual_level(), torch.set_grad_enabled(grad_mode):
+        if dual == "w":
+            w = fwAD.make_dual(w, torch.ones_like(w))
+        else:
+            a = fwAD.make_dual(a, torch.ones_like(a))
+        if "cached" in dual:
+            w, _ = create_quantized_weight(w, E4, _config(gran))
+        with pytest.raises((NotImplementedError, RuntimeError), match="(?i)jvp|forward mode|forward AD" if "cached" not in dual else None):
+            op(a, w)
 
 
 # ---- weights quantised ahead of time ----------------------------------------------------------------------------
