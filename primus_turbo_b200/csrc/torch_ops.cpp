@@ -11,6 +11,7 @@
 // frozen weights) are not computed.  Every entry returns None when an argument is not the plain case handled
 // here, and the Python form -- with its checks, its error messages and its per-kernel instrumentation -- takes over.
 #include <ATen/ATen.h>
+#include <ATen/TracerMode.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -614,6 +615,10 @@ template <typename F> py::object guarded(F &&f) {
 // looks like inference: the Python form raises, here the tangent would be dropped.
 bool has_tangent(const Tensor &t) { return t._fw_grad(/*level=*/0).defined(); }
 
+// torch.jit.trace records the Python form as an op that runs again on new inputs; a call from here would leave nothing in the
+// trace but its output, as a constant.
+bool traced() { return at::tracer::impl::is_dispatch_enabled(); }
+
 bool plain_cuda(const Tensor &t) { return t.device().is_cuda() && t.layout() == at::kStrided && t.numel() > 0; }
 
 // The scales of a weight [.., rows, cols] quantised ahead of time: as the kernels read them, and as many.  Anything else -- another
@@ -633,7 +638,7 @@ bool scales_fit(const Tensor &w, const Tensor &s, int gran, bool tb) {
 
 py::object py_gemm_fp8(const Tensor &a, const Tensor &b, const std::optional<Tensor> &b_scale, bool ta, bool tb, ScalarType out,
                        int gran, ScalarType fwd, ScalarType bwd) {
-    if (has_tangent(a) || has_tangent(b)) return py::none();
+    if (traced() || has_tangent(a) || has_tangent(b)) return py::none();
     if (!plain_cuda(a) || !plain_cuda(b) || a.device() != b.device() || a.dim() != 2 || b.dim() != 2 || !is_hp(a.scalar_type()) ||
         !is_hp(out) || a.size(ta ? 0 : 1) != b.size(tb ? 1 : 0))
         return py::none();
@@ -657,7 +662,7 @@ py::object py_gemm_fp8(const Tensor &a, const Tensor &b, const std::optional<Ten
 py::object py_grouped_gemm_fp8(const Tensor &a, const Tensor &b, const std::optional<Tensor> &b_scale, const Tensor &lens,
                                const std::optional<Tensor> &offs, bool tb, ScalarType out, int gran, ScalarType fwd, ScalarType bwd,
                                int num_sms) {
-    if (has_tangent(a) || has_tangent(b)) return py::none();
+    if (traced() || has_tangent(a) || has_tangent(b)) return py::none();
     if (!plain_cuda(a) || !plain_cuda(b) || !plain_cuda(lens) || a.device() != b.device() || a.device() != lens.device() ||
         a.dim() != 2 || b.dim() != 3 || !is_hp(a.scalar_type()) || !is_16bit(out) || a.size(1) != b.size(tb ? 2 : 1) ||
         lens.dim() != 1 || lens.scalar_type() != ScalarType::Long || lens.size(0) != b.size(0) || !lens.is_contiguous())
@@ -689,7 +694,7 @@ bool quantisable(const Tensor &x) {
 
 // kind: the granularity; BLOCKWISE with tiles = 128x128 scales.  -> (q, scale_inv)
 py::object py_quantize(const Tensor &x, ScalarType dt, int gran, int64_t axis, bool tiles) {
-    if (!quantisable(x) || !is_fp8(dt)) return py::none();
+    if (traced() || !quantisable(x) || !is_fp8(dt)) return py::none();
     const int64_t nd = x.dim();
     if (gran == PTB_ROWWISE && (nd == 0 || axis < 0 || axis >= nd)) return py::none();
     if (gran == PTB_BLOCKWISE && (tiles ? nd != 2 && nd != 3 : nd != 2 || axis < 0 || axis > 1)) return py::none();
@@ -718,7 +723,7 @@ py::object py_quantize(const Tensor &x, ScalarType dt, int gran, int64_t axis, b
 
 // -> (row copy, row scales, column copy, column scales)
 py::object py_quantize_dual(const Tensor &x, ScalarType dt, int gran, bool row_2d, bool col_2d) {
-    if (!quantisable(x) || !is_fp8(dt)) return py::none();
+    if (traced() || !quantisable(x) || !is_fp8(dt)) return py::none();
     const int64_t nd = x.dim();
     if (gran == PTB_BLOCKWISE ? nd != 2 : (nd != 2 && nd != 3) || !is_16bit(x.scalar_type()) || x.size(-1) % kMxBlk) return py::none();
     return guarded([&]() -> py::object {
@@ -733,7 +738,7 @@ py::object py_quantize_dual(const Tensor &x, ScalarType dt, int gran, bool row_2
 }
 
 py::object py_dequantize(const Tensor &q, const Tensor &s, ScalarType out_dt, int gran, int64_t axis, bool tiles) {
-    if (!plain_cuda(q) || !plain_cuda(s) || q.device() != s.device() || !is_fp8(q.scalar_type()) || !is_hp(out_dt) ||
+    if (traced() || !plain_cuda(q) || !plain_cuda(s) || q.device() != s.device() || !is_fp8(q.scalar_type()) || !is_hp(out_dt) ||
         !q.is_contiguous() || !s.is_contiguous())
         return py::none();
     const int64_t nd = q.dim();

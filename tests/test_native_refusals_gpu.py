@@ -57,6 +57,21 @@ def test_a_forward_mode_tangent_is_refused(gran, grouped, dual, grad_mode):
             op(a, w)
 
 
+# ---- torch.jit.trace --------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("grouped", [False, True])
+@pytest.mark.parametrize("gran", GRANS)
+def test_a_traced_call_runs_again_on_new_inputs(gran, grouped):
+    op, a, w = _op(grouped, gran)
+    other = _rand(100, 256, seed=7)
+    if gran == G.MX_BLOCKWISE:  # torch cannot record the byte views of the MX form: an error, not a constant
+        with pytest.raises(RuntimeError):
+            torch.jit.trace(lambda x: op(x, w), (a,), check_trace=False)
+        return
+    traced = torch.jit.trace(lambda x: op(x, w), (a,), check_trace=False)
+    assert torch.equal(traced(other), op(other, w))
+    assert torch.equal(traced(a), op(a, w))
+
+
 # ---- weights quantised ahead of time ----------------------------------------------------------------------------
 def _with_scale(q, scale):
     return QuantizedTensor(q.qdata, scale, shape=q.shape, orig_dtype=q.dtype, dest_dtype=q.real_dtype, granularity=q.granularity,
