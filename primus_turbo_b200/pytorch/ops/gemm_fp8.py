@@ -231,11 +231,13 @@ class FP8GemmMXFunction(torch.autograd.Function):
 _TILES = ScalingRecipe(use_2d_block=True)  # how BLOCKWISE and MX weights are quantised
 
 
-def _native_gemm(a, b, trans_a, trans_b, out_dtype, config):
+def _native_gemm(a, b, a_t, b_t, trans_a, trans_b, out_dtype, config):
     """The whole call through the native host path; ``None`` where it has to run in Python."""
     g = config.granularity
     if g == ScalingGranularity.BLOCKWISE and config.block_size != 128:
         return None
+    if a_t is not None or (b_t is not None and not (isinstance(b, QuantizedTensor) and isinstance(b_t, QuantizedTensor))):
+        return None  # a copy for the backward pass beside a raw operand
     b_scale = None
     if isinstance(b, QuantizedTensor):
         # a weight quantised ahead of time, in inference: its payload in the forward direction is all that is read
@@ -246,6 +248,8 @@ def _native_gemm(a, b, trans_a, trans_b, out_dtype, config):
             ok = ok and b.quantized_axis == (1 if trans_b else 0)
         if not ok or b.requires_grad or (a.requires_grad and torch.is_grad_enabled()):
             return None
+        if g == ScalingGranularity.MX_BLOCKWISE and b_t is not None:
+            check_quantized_tensor(b_t, config, axis=-2, scaling_recipe=_TILES)
         b, b_scale = b.qdata, b.scale_inv
     elif not _native.usable(b):
         return None
@@ -275,7 +279,7 @@ def gemm_fp8(
     if out_dtype is None:
         out_dtype = torch.promote_types(a_data.dtype, b_data.dtype)
     if _native.usable(a_data):
-        out = _native_gemm(a_data, b_data, trans_a, trans_b, out_dtype, config)
+        out = _native_gemm(a_data, b_data, a_data_t, b_data_t, trans_a, trans_b, out_dtype, config)
         if out is not None:
             return out
     return _gemm_fp8_python(a_data, b_data, a_data_t, b_data_t, trans_a, trans_b, out_dtype, config)

@@ -302,11 +302,13 @@ class FP8GroupedGemmMXFunc(torch.autograd.Function):
         return grad_a, grad_b, None, None, None, None, None, None, None, None
 
 
-def _native_grouped(a, b, group_lens, group_offs, trans_b, out_dtype, config, num_cu):
+def _native_grouped(a, b, a_t, b_t, group_lens, group_offs, trans_b, out_dtype, config, num_cu):
     """The whole call through the native host path; ``None`` where it has to run in Python."""
     g = config.granularity
     if g == ScalingGranularity.BLOCKWISE and config.block_size != 128:
         return None
+    if a_t is not None or (b_t is not None and not (isinstance(b, QuantizedTensor) and isinstance(b_t, QuantizedTensor))):
+        return None  # a copy for the backward pass beside a raw operand
     b_scale = None
     fwd = _get_fp8_dtype(config.format, True)
     if isinstance(b, QuantizedTensor):
@@ -318,6 +320,8 @@ def _native_grouped(a, b, group_lens, group_offs, trans_b, out_dtype, config, nu
             ok = ok and b.quantized_axis == (2 if trans_b else 1)
         if not ok or b.requires_grad or (a.requires_grad and torch.is_grad_enabled()):
             return None
+        if g == ScalingGranularity.MX_BLOCKWISE and b_t is not None:
+            check_quantized_tensor(b_t, config, axis=-2, scaling_recipe=_WEIGHT_RECIPE)
         b, b_scale = b.qdata, b.scale_inv
     elif not _native.usable(b):
         return None
@@ -348,7 +352,7 @@ def grouped_gemm_fp8(
     if out_dtype is None:
         out_dtype = torch.promote_types(a_data.dtype, b_data.dtype)
     if _native.usable(a_data):
-        out = _native_grouped(a_data, b_data, group_lens, group_offs, trans_b, out_dtype, config, num_cu)
+        out = _native_grouped(a_data, b_data, a_data_t, b_data_t, group_lens, group_offs, trans_b, out_dtype, config, num_cu)
         if out is not None:
             return out
     if group_offs is None:

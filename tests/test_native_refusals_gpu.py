@@ -7,7 +7,7 @@ import torch.autograd.forward_ad as fwAD
 
 from primus_turbo_b200.pytorch.core.low_precision import Float8QuantConfig, Format, ScaleDtype
 from primus_turbo_b200.pytorch.core.low_precision import ScalingGranularity as G
-from primus_turbo_b200.pytorch.core.quantized_tensor import QuantizedTensor, create_quantized_weight
+from primus_turbo_b200.pytorch.core.quantized_tensor import QuantizedTensor, QuantizedTensorPair, create_quantized_weight
 from primus_turbo_b200.pytorch.ops import gemm_fp8, grouped_gemm_fp8
 
 pytestmark = pytest.mark.gpu
@@ -95,3 +95,33 @@ def test_a_cached_weight_with_wider_scales_is_still_taken(gran, grouped):
     q, _ = create_quantized_weight(w, E4, _config(gran))
     with torch.no_grad():
         assert torch.equal(op(a, _with_scale(q, q.scale_inv.double())), op(a, q))
+
+
+# ---- operands that come as a pair ------------------------------------------------------------------------------------
+@pytest.mark.parametrize("gran", [G.ROWWISE, G.MX_BLOCKWISE])
+@pytest.mark.parametrize("grouped", [False, True])
+def test_a_companion_that_does_not_fit_is_refused(gran, grouped):
+    """The backward-direction copy of a pair is checked in inference as well, as the Python form does."""
+    op, a, w = _op(grouped, gran)
+    q, q_t = create_quantized_weight(w, E4, _config(gran), need_weight_transpose_cache=True)
+    with torch.no_grad():
+        assert torch.equal(op(a, QuantizedTensorPair(q, q_t)), op(a, q))
+        with pytest.raises((AssertionError, AttributeError)):
+            op(a, QuantizedTensorPair(q, w))
+        if gran == G.MX_BLOCKWISE:
+            with pytest.raises(AssertionError):
+                op(a, QuantizedTensorPair(q, q))
+
+
+@pytest.mark.parametrize("which", ["a", "w"])
+def test_a_companion_beside_a_raw_operand_is_used(which):
+    """ROWWISE: the copy handed in for the backward pass is the one the gradient is made from."""
+    op, a, w = _op(False, G.ROWWISE)
+    a.requires_grad_(), w.requires_grad_()
+    a_t = QuantizedTensor.quantize(torch.zeros_like(a), E4, G.ROWWISE, axis=-2)
+    w_t = QuantizedTensor.quantize(torch.zeros_like(w), E4, G.ROWWISE, axis=-2)
+    pair = (QuantizedTensorPair(a, a_t), w) if which == "a" else (a, QuantizedTensorPair(w, w_t))
+    out = op(*pair)
+    ga, gw = torch.autograd.grad(out, (a, w), torch.ones_like(out))
+    zero, other = (gw, ga) if which == "a" else (ga, gw)
+    assert not zero.any() and other.any()
