@@ -326,7 +326,7 @@ def _native_grouped(a, b, a_t, b_t, group_lens, group_offs, trans_b, out_dtype, 
     elif not _native.usable(b):
         return None
     return _native.ext.grouped_gemm_fp8(a, b, b_scale, group_lens, group_offs, trans_b, out_dtype, g.value, fwd,
-                                        _get_fp8_dtype(config.format, False), num_cu or 0)
+                                        _get_fp8_dtype(config.format, False), int(num_cu or 0))
 
 
 def grouped_gemm_fp8(

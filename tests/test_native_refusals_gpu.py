@@ -125,3 +125,10 @@ def test_a_companion_beside_a_raw_operand_is_used(which):
     ga, gw = torch.autograd.grad(out, (a, w), torch.ones_like(out))
     zero, other = (gw, ga) if which == "a" else (ga, gw)
     assert not zero.any() and other.any()
+
+
+# ---- the SM cap ------------------------------------------------------------------------------------------------------
+def test_num_cu_may_be_any_number():
+    a, w, lens = _rand(100, 256), _rand(3, 384, 256, seed=2), torch.tensor(LENS, device=DEV)
+    with torch.no_grad():
+        assert torch.equal(grouped_gemm_fp8(a, w, lens, num_cu=8.0), grouped_gemm_fp8(a, w, lens, num_cu=8))
