@@ -743,8 +743,8 @@ py::object py_dequantize(const Tensor &q, const Tensor &s, ScalarType out_dt, in
         return py::none();
     const int64_t nd = q.dim();
     const bool f32 = s.scalar_type() == ScalarType::Float;
-    if (gran == kMxGranularity ? nd != 2 || axis < 0 || axis > 1 || q.size(1) % kMxBlk || s.dim() != 2 || s.element_size() != 1
-                               : !f32)
+    const bool e8m0 = s.scalar_type() == ScalarType::Float8_e8m0fnu || s.scalar_type() == ScalarType::Byte;
+    if (gran == kMxGranularity ? nd != 2 || axis < 0 || axis > 1 || q.size(1) % kMxBlk || s.dim() != 2 || !e8m0 : !f32)
         return py::none();
     if (gran == PTB_ROWWISE && (nd == 0 || axis < 0 || axis >= nd)) return py::none();
     if (gran == PTB_BLOCKWISE && (tiles ? nd != 2 && nd != 3 : nd != 2 || axis < 0 || axis > 1)) return py::none();

@@ -8,7 +8,7 @@ import torch.autograd.forward_ad as fwAD
 from primus_turbo_b200.pytorch.core.low_precision import Float8QuantConfig, Format, ScaleDtype
 from primus_turbo_b200.pytorch.core.low_precision import ScalingGranularity as G
 from primus_turbo_b200.pytorch.core.quantized_tensor import QuantizedTensor, QuantizedTensorPair, create_quantized_weight
-from primus_turbo_b200.pytorch.ops import gemm_fp8, grouped_gemm_fp8
+from primus_turbo_b200.pytorch.ops import dequantize_fp8, gemm_fp8, grouped_gemm_fp8, quantize_fp8
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -132,3 +132,15 @@ def test_num_cu_may_be_any_number():
     a, w, lens = _rand(100, 256), _rand(3, 384, 256, seed=2), torch.tensor(LENS, device=DEV)
     with torch.no_grad():
         assert torch.equal(grouped_gemm_fp8(a, w, lens, num_cu=8.0), grouped_gemm_fp8(a, w, lens, num_cu=8))
+
+
+# ---- dequantise -------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("axis", [0, 1])
+def test_mx_scales_of_another_byte_type_are_refused(axis):
+    q, s = quantize_fp8(_rand(128, 256), E4, G.MX_BLOCKWISE, block_size=32, axis=axis)
+    kw = dict(block_size=32, axis=axis)
+    y = dequantize_fp8(q, torch.bfloat16, G.MX_BLOCKWISE, scale_inv=s, **kw)
+    assert torch.equal(dequantize_fp8(q, torch.bfloat16, G.MX_BLOCKWISE, scale_inv=s.view(torch.uint8), **kw), y)
+    for other in (torch.int8, E4, torch.float8_e5m2):
+        with pytest.raises(AssertionError, match="e8m0"):
+            dequantize_fp8(q, torch.bfloat16, G.MX_BLOCKWISE, scale_inv=s.view(other), **kw)
