@@ -30,7 +30,7 @@ template <> struct MxFmt<PTB_E5M2> { static constexpr int mbits = 2, target_pow2
 
 // Block maximum -> biased E8M0 byte.  The maximum's mantissa is rounded to the FP8 format's width (the
 // carry may bump the exponent), the exponent of the format's largest power of two is subtracted, the
-// result is clamped to [-127, 128] and biased by 127.  A maximum is never negative and at most infinity, so the biased
+// result is clamped to [-127, 128] and biased by 127.  A maximum is never negative, never NaN and at most infinity, so the biased
 // exponent before the subtraction is at most 255 and only the lower clamp can bind.
 template <int FMT, bool ZERO_IS_ONE> __device__ __forceinline__ int mx_byte(float amax) {
     if (ZERO_IS_ONE && amax == 0.0f) return 127;
@@ -221,7 +221,8 @@ __global__ void __launch_bounds__(256, PTB_MXQ_MINB) mx_quant_kernel(const MxQua
                 cm[3] = max2<T>(cm[3], a3);
                 m[k]  = max2<T>(max2<T>(a0, a1), max2<T>(a2, a3));
             }
-            const uint32_t both = max2<T>(__byte_perm(m[0], m[1], 0x5410), __byte_perm(m[0], m[1], 0x7632));
+            // from zero, like the column maxima: a maximum passes over NaN also where a lane holds nothing else
+            const uint32_t both = max2<T>(max2<T>(0u, __byte_perm(m[0], m[1], 0x5410)), __byte_perm(m[0], m[1], 0x7632));
             rm[i]               = shfl_max2<T>(shfl_max2<T>(both, 1), 2); // the four lanes of a 32-column block
         }
 #pragma unroll
