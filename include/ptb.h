@@ -5,13 +5,13 @@
  * (passed as void*, i.e. a cudaStream_t).  The caller allocates every output and workspace.  All
  * work is enqueued on the given stream; no call synchronises the host with the device (except
  * ptb_gemm_status and ptb_copy_segments_status, which read one word back).  Calls are re-entrant.
- * The library keeps no state between calls, with three stated exceptions:
+ * The library keeps no state between calls, with four stated exceptions:
  * (1) ptb_quant_fp8_rowwise_noalloc reduces into one fixed device array that all of its calls
  * share; (2) the GEMM kernels record a wait that ran out
  * in one device word per GPU, shared by all streams and read with ptb_gemm_status, and the peer
  * copies do the same for a bad rank number or a flag wait that ran out (ptb_copy_segments_status);
  * (3) per-device one-time set-up (kernel attributes, the address of that array) is cached in the
- * process.
+ * process; (4) a running count of the kernels enqueued (ptb_kernels_enqueued).
  *
  * Alignment: FP8 outputs of the blockwise quantise entry points (block1d, block1d_dual, block2d,
  * segment_row_col) must be 8-byte aligned, GEMM operands 16-byte aligned with leading dimensions
@@ -60,6 +60,10 @@ typedef void *ptb_stream_t; /* cudaStream_t */
 
 int ptb_version(void);
 const char *ptb_last_error(void);
+
+/* Kernels this process has enqueued through the library so far, all threads and devices together (memsets not counted): each
+ * is counted where it is launched. */
+int64_t ptb_kernels_enqueued(void);
 
 /* ------------------------------------------------------------------ quantize ----------------- */
 

@@ -79,7 +79,7 @@ _PROTOS = {
     "ptb_gemm_wait_selftest": [_P],
 }
 
-EXPORTS = ["ptb_version", "ptb_last_error", *_PROTOS.keys()]
+EXPORTS = ["ptb_version", "ptb_last_error", "ptb_kernels_enqueued", *_PROTOS.keys()]
 
 
 def _load() -> ctypes.CDLL:
@@ -93,6 +93,8 @@ def _load() -> ctypes.CDLL:
     lib.ptb_version.argtypes = []
     lib.ptb_last_error.restype = c_char_p
     lib.ptb_last_error.argtypes = []
+    lib.ptb_kernels_enqueued.restype = ctypes.c_int64
+    lib.ptb_kernels_enqueued.argtypes = []
     for name, args in _PROTOS.items():
         fn = getattr(lib, name)
         fn.restype = c_int
@@ -113,11 +115,6 @@ def check(rc: int, what: str) -> None:
         raise PtbError(f"{what} failed with status {rc}: {msg}")
 
 
-# kernels enqueued by one successful call of each entry point (memset nodes not counted; a tensorwise quantise of at most
-# 262144 elements is one, not two)
-KERNELS_PER_CALL = {"ptb_quant_fp8_tensorwise": 2, "ptb_quant_fp8_rowwise": 2, "ptb_quant_fp8_rowwise_noalloc": 2, "ptb_requant_fp8_rowwise": 2,
-                    "ptb_quant_fp8_segment_row_col": 2, "ptb_quant_mxfp8_grouped": 2, "ptb_moe_row_id_map": 3, "ptb_swiglu_quant_fp8_segment_row_col": 2,
-                    "ptb_gemm_status": 0, "ptb_copy_segments_status": 0, "ptb_enable_peer_access": 0}
 # PTB_DEBUG_STATUS=1: after every GEMM call, wait for the device and raise if a bounded wait inside the
 # kernel ran out (status codes in include/ptb.h).  Off by default: the check synchronises.
 _DEBUG_STATUS = os.environ.get("PTB_DEBUG_STATUS", "0") not in ("", "0")
@@ -125,15 +122,12 @@ _GEMM_ENTRY_POINTS = ("ptb_gemm_fp8", "ptb_gemm_mxfp8", "ptb_grouped_gemm_fp8", 
                       "ptb_grouped_gemm_mxfp8", "ptb_grouped_gemm_mxfp8_variable_k")
 # PTB_NVTX=1: one NVTX range per C-ABI call, named after the entry point (timeline tools show them)
 _NVTX = os.environ.get("PTB_NVTX", "0") not in ("", "0")
-_launches = 0  # kernels enqueued by ``call``
-_native_launches = lambda: 0  # noqa: E731  (kernels enqueued by the native host path, once that is loaded)
 _event_log = None  # when a dict: name -> [(start_event, stop_event), ...] on the launching stream
 
 
 def call(name: str, *args) -> None:
-    """Invoke one C-ABI entry point: count its launches, optionally bracket it with CUDA events on
-    the current stream (see record_kernel_times), raise PtbError on a non-zero status."""
-    global _launches
+    """Invoke one C-ABI entry point: optionally bracket it with CUDA events on the current stream (see
+    record_kernel_times), raise PtbError on a non-zero status."""
     fn = getattr(lib, name)
     if _NVTX:
         torch.cuda.nvtx.range_push(name)
@@ -142,7 +136,6 @@ def call(name: str, *args) -> None:
         finally:
             torch.cuda.nvtx.range_pop()
         check(rc, name)
-        _launches += KERNELS_PER_CALL.get(name, 1)
         return
     if _event_log is not None:
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -153,7 +146,6 @@ def call(name: str, *args) -> None:
     else:
         rc = fn(*args)
     check(rc, name)
-    _launches += KERNELS_PER_CALL.get(name, 1)
     if _DEBUG_STATUS and name in _GEMM_ENTRY_POINTS and not torch.cuda.is_current_stream_capturing():
         # (a stream that is being captured into a graph cannot be waited for: the check is skipped there)
         torch.cuda.synchronize()
@@ -163,8 +155,8 @@ def call(name: str, *args) -> None:
 
 
 def __getattr__(name: str):
-    if name == "launch_count":  # running total of kernels this process enqueued through the C ABI
-        return _launches + _native_launches()
+    if name == "launch_count":  # running total of kernels this process enqueued through the C ABI, by whichever host path
+        return lib.ptb_kernels_enqueued()
     raise AttributeError(name)
 
 

@@ -30,7 +30,6 @@ def _load():
 
 
 ext = _load()
-_lib._native_launches = ext.launches
 _PLAIN = (torch.Tensor, torch.nn.Parameter)
 
 

@@ -43,10 +43,14 @@ inline int cuda_fail(cudaError_t e, const char *where) {
         if (_e != cudaSuccess) return ::ptb::cuda_fail(_e, #expr);    \
     } while (0)
 
+void count_kernel(); // one more kernel enqueued by this process (ptb_kernels_enqueued)
+
+// after every kernel launch, once
 #define PTB_LAUNCH_CHECK(name)                                        \
     do {                                                              \
         cudaError_t _e = cudaGetLastError();                          \
         if (_e != cudaSuccess) return ::ptb::cuda_fail(_e, name);     \
+        ::ptb::count_kernel();                                        \
     } while (0)
 
 inline bool is_fp8(int dt) { return dt == PTB_E4M3 || dt == PTB_E5M2; }

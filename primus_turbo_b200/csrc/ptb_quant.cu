@@ -12,6 +12,8 @@ namespace ptb {
 
 thread_local char g_err[kErrBufLen] = {0};
 char *err_buf() { return g_err; }
+std::atomic<int64_t> g_kernels{0};
+void count_kernel() { g_kernels.fetch_add(1, std::memory_order_relaxed); }
 
 namespace {
 
@@ -1287,6 +1289,7 @@ extern "C" {
 
 int ptb_version(void) { return PTB_VERSION; }
 const char *ptb_last_error(void) { return err_buf(); }
+int64_t ptb_kernels_enqueued(void) { return g_kernels.load(std::memory_order_relaxed); }
 
 int ptb_quant_fp8_tensorwise(const void *x, int x_dtype, int64_t n, void *q, int q_dtype, float *scale_inv,
                              void *workspace, ptb_stream_t stream) {

@@ -38,7 +38,7 @@ namespace {
 constexpr int kMxGranularity = 4; // ScalingGranularity.MX_BLOCKWISE
 constexpr int64_t kBlk = 128, kMxBlk = 32;
 
-std::atomic<int64_t> g_launches{0};
+std::atomic<int64_t> g_calls{0}; // C-ABI calls that enqueued work from here
 std::atomic<bool> g_check_status{false}; // debug: wait for the device after every GEMM and read the status word
 PyObject *g_error_class = nullptr;
 
@@ -46,19 +46,19 @@ struct PtbFail : std::runtime_error {
     using std::runtime_error::runtime_error;
 };
 
-void check(int rc, const char *what, int kernels) {
+void check(int rc, const char *what) {
     if (rc != 0) throw PtbFail(std::string(what) + " failed with status " + std::to_string(rc) + ": " + ptb_last_error());
-    g_launches.fetch_add(kernels, std::memory_order_relaxed);
+    g_calls.fetch_add(1, std::memory_order_relaxed);
 }
 
 void check_gemm(int rc, const char *what, cudaStream_t st) {
-    check(rc, what, 1);
+    check(rc, what);
     if (!g_check_status.load(std::memory_order_relaxed)) return;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return;
     cudaDeviceSynchronize();
     int code = 0;
-    check(ptb_gemm_status(&code, 1), "ptb_gemm_status", 0);
+    check(ptb_gemm_status(&code, 1), "ptb_gemm_status");
     if (code != 0)
         throw PtbFail(std::string(what) + ": a device-side wait ran out (status " + std::to_string(code) +
                       "); the output is incomplete");
@@ -108,7 +108,7 @@ Quant quant_tensorwise(const Call &c, const Tensor &x, ScalarType dt) {
     Tensor ws = c.empty({PTB_TENSORWISE_WS_BYTES}, ScalarType::Byte);
     check(ptb_quant_fp8_tensorwise(x.const_data_ptr(), code_of(x.scalar_type()), x.numel(), r.q.mutable_data_ptr(), code_of(dt),
                                    r.s.mutable_data_ptr<float>(), ws.mutable_data_ptr(), c.st),
-          "ptb_quant_fp8_tensorwise", 2);
+          "ptb_quant_fp8_tensorwise");
     return r;
 }
 
@@ -126,7 +126,7 @@ Quant quant_rowwise(const Call &c, const Tensor &x, ScalarType dt, int64_t axis)
     if (N > 1) ws = c.empty({B * N}, ScalarType::Float);
     check(ptb_quant_fp8_rowwise(x.const_data_ptr(), code_of(x.scalar_type()), B, M, N, r.q.mutable_data_ptr(), code_of(dt),
                                 r.s.mutable_data_ptr<float>(), N > 1 ? ws.mutable_data_ptr() : nullptr, c.st),
-          "ptb_quant_fp8_rowwise", N > 1 ? 2 : 1);
+          "ptb_quant_fp8_rowwise");
     return r;
 }
 
@@ -138,7 +138,7 @@ Tensor dequant_rowwise(const Call &c, const Tensor &q, const Tensor &s, ScalarTy
     Tensor out = c.empty(q.sizes(), dt);
     check(ptb_dequant_fp8_rowwise(q.const_data_ptr(), code_of(q.scalar_type()), B, q.size(axis), N, s.const_data_ptr<float>(),
                                   out.mutable_data_ptr(), code_of(dt), c.st),
-          "ptb_dequant_fp8_rowwise", 1);
+          "ptb_dequant_fp8_rowwise");
     return out;
 }
 
@@ -156,7 +156,7 @@ Quant requant_rowwise(const Call &c, const Quant &r, ScalarType hp, int64_t have
     Tensor ws = c.empty({B * N}, ScalarType::Float);
     check(ptb_requant_fp8_rowwise(r.q.const_data_ptr(), code_of(r.q.scalar_type()), r.scale(), code_of(hp), B, M, N,
                                   o.q.mutable_data_ptr(), o.s.mutable_data_ptr<float>(), ws.mutable_data_ptr(), c.st),
-          "ptb_requant_fp8_rowwise", 2);
+          "ptb_requant_fp8_rowwise");
     return o;
 }
 
@@ -165,7 +165,7 @@ Quant quant_block_rows(const Call &c, const Tensor &x, ScalarType dt) {
     Quant r{c.empty({M, N}, dt), c.empty({M, nb}, ScalarType::Float), nb, 1};
     check(ptb_quant_fp8_block1d(x.const_data_ptr(), code_of(x.scalar_type()), M, N, 1, r.q.mutable_data_ptr(), code_of(dt),
                                 r.s.mutable_data_ptr<float>(), c.st),
-          "ptb_quant_fp8_block1d", 1);
+          "ptb_quant_fp8_block1d");
     return r;
 }
 
@@ -174,7 +174,7 @@ Quant quant_block_cols(const Call &c, const Tensor &x, ScalarType dt) {
     Quant r{c.empty({M, N}, dt), c.empty({cdiv(M, kBlk), N}, ScalarType::Float), 1, N};
     check(ptb_quant_fp8_block1d(x.const_data_ptr(), code_of(x.scalar_type()), M, N, 0, r.q.mutable_data_ptr(), code_of(dt),
                                 r.s.mutable_data_ptr<float>(), c.st),
-          "ptb_quant_fp8_block1d", 1);
+          "ptb_quant_fp8_block1d");
     return r;
 }
 
@@ -185,7 +185,7 @@ std::pair<Quant, Quant> quant_block_dual(const Call &c, const Tensor &x, ScalarT
     check(ptb_quant_fp8_block1d_dual(x.const_data_ptr(), code_of(x.scalar_type()), M, N, row.q.mutable_data_ptr(),
                                      row.s.mutable_data_ptr<float>(), col.q.mutable_data_ptr(), col.s.mutable_data_ptr<float>(),
                                      code_of(dt), c.st),
-          "ptb_quant_fp8_block1d_dual", 1);
+          "ptb_quant_fp8_block1d_dual");
     return {row, col};
 }
 
@@ -197,7 +197,7 @@ Quant quant_block_tiles(const Call &c, const Tensor &w, ScalarType dt) {
             nb, 1, mb * nb};
     check(ptb_quant_fp8_block2d(w.const_data_ptr(), code_of(w.scalar_type()), B, M, N, r.q.mutable_data_ptr(), code_of(dt),
                                 r.s.mutable_data_ptr<float>(), c.st),
-          "ptb_quant_fp8_block2d", 1);
+          "ptb_quant_fp8_block2d");
     return r;
 }
 
@@ -216,7 +216,7 @@ std::pair<Quant, Quant> quant_mx(const Call &c, const Tensor &x, ScalarType dt, 
     check(ptb_quant_mxfp8(x.const_data_ptr(), code_of(x.scalar_type()), G, M, N, want_row ? row.q.mutable_data_ptr() : nullptr,
                           want_row ? row.s.mutable_data_ptr() : nullptr, want_col ? col.q.mutable_data_ptr() : nullptr,
                           want_col ? col.s.mutable_data_ptr() : nullptr, row_2d, col_2d, code_of(dt), c.st),
-          "ptb_quant_mxfp8", 1);
+          "ptb_quant_mxfp8");
     return {row, col};
 }
 
@@ -349,7 +349,7 @@ struct Layout {
 
 Tensor group_offsets(const Call &c, const Tensor &lens) {
     Tensor offs = c.empty({lens.numel() + 1}, ScalarType::Long);
-    check(ptb_group_offs(lens.const_data_ptr<int64_t>(), lens.numel(), offs.mutable_data_ptr<int64_t>(), c.st), "ptb_group_offs", 1);
+    check(ptb_group_offs(lens.const_data_ptr<int64_t>(), lens.numel(), offs.mutable_data_ptr<int64_t>(), c.st), "ptb_group_offs");
     return offs;
 }
 
@@ -365,7 +365,7 @@ std::pair<Quant, Quant> quant_segments(const Call &c, const Tensor &x, ScalarTyp
                                         l.offs.const_data_ptr<int64_t>(), row.q.mutable_data_ptr(), col.q.mutable_data_ptr(),
                                         row.s.mutable_data_ptr<float>(), col.s.mutable_data_ptr<float>(), p + G + 1, p,
                                         table.mutable_data_ptr(), code_of(dt), c.st),
-          "ptb_quant_fp8_segment_row_col", 2);
+          "ptb_quant_fp8_segment_row_col");
     l.padded = pads; // first G + 1 words: the padded offsets
     return {row, col};
 }
@@ -381,7 +381,7 @@ std::pair<Quant, Quant> quant_mx_groups(const Call &c, const Tensor &x, ScalarTy
                                   row.q.mutable_data_ptr(), row.s.mutable_data_ptr(), col.q.mutable_data_ptr(),
                                   col.s.mutable_data_ptr(), p + G + 1, p + 2 * G + 1, p + 3 * G + 2, p, table.mutable_data_ptr(),
                                   0, 0, code_of(dt), c.st),
-          "ptb_quant_mxfp8_grouped", 2);
+          "ptb_quant_mxfp8_grouped");
     l.padded = pads;
     return {row, col};
 }
@@ -758,21 +758,21 @@ py::object py_dequantize(const Tensor &q, const Tensor &s, ScalarType out_dt, in
         switch (gran) {
         case PTB_TENSORWISE:
             check(ptb_dequant_fp8_tensorwise(q.const_data_ptr(), qc, q.numel(), s.const_data_ptr<float>(), o, oc, c.st),
-                  "ptb_dequant_fp8_tensorwise", 1);
+                  "ptb_dequant_fp8_tensorwise");
             break;
         case PTB_BLOCKWISE:
             if (tiles)
                 check(ptb_dequant_fp8_block2d(q.const_data_ptr(), qc, nd == 3 ? q.size(0) : 1, q.size(-2), q.size(-1),
                                               s.const_data_ptr<float>(), o, oc, c.st),
-                      "ptb_dequant_fp8_block2d", 1);
+                      "ptb_dequant_fp8_block2d");
             else
                 check(ptb_dequant_fp8_block1d(q.const_data_ptr(), qc, q.size(0), q.size(1), axis == 1,
                                               s.const_data_ptr<float>(), o, oc, c.st),
-                      "ptb_dequant_fp8_block1d", 1);
+                      "ptb_dequant_fp8_block1d");
             break;
         default:
             check(ptb_dequant_mxfp8(q.const_data_ptr(), qc, q.size(0), q.size(1), s.const_data_ptr(), flip, o, oc, c.st),
-                  "ptb_dequant_mxfp8", 1);
+                  "ptb_dequant_mxfp8");
         }
         return py::cast(out);
     });
@@ -786,7 +786,7 @@ PYBIND11_MODULE(ptb_torch, m) {
         g_error_class = error_class.release().ptr(); // kept for the life of the process
         g_check_status = check_status;
     });
-    m.def("launches", [] { return g_launches.load(std::memory_order_relaxed); });
+    m.def("calls", [] { return g_calls.load(std::memory_order_relaxed); });
     m.def("gemm_fp8", &py_gemm_fp8);
     m.def("grouped_gemm_fp8", &py_grouped_gemm_fp8);
     m.def("quantize", &py_quantize);

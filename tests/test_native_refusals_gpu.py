@@ -5,6 +5,7 @@ import pytest
 import torch
 import torch.autograd.forward_ad as fwAD
 
+from primus_turbo_b200 import _lib
 from primus_turbo_b200.pytorch.core.low_precision import Float8QuantConfig, Format, ScaleDtype
 from primus_turbo_b200.pytorch.core.low_precision import ScalingGranularity as G
 from primus_turbo_b200.pytorch.core.quantized_tensor import QuantizedTensor, QuantizedTensorPair, create_quantized_weight
@@ -70,6 +71,31 @@ def test_a_traced_call_runs_again_on_new_inputs(gran, grouped):
     traced = torch.jit.trace(lambda x: op(x, w), (a,), check_trace=False)
     assert torch.equal(traced(other), op(other, w))
     assert torch.equal(traced(a), op(a, w))
+
+
+# ---- kernel counts ----------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("recorded", [False, True])
+@pytest.mark.parametrize("n,offset,dtype,kernels", [
+    (262144, 0, torch.bfloat16, 1), (8, 0, torch.float16, 1), (262152, 0, torch.bfloat16, 2), (262140, 0, torch.bfloat16, 2),
+    (4096, 1, torch.bfloat16, 2), (4096, 0, torch.float32, 2),
+])
+def test_tensorwise_quantise_counts_the_kernels_it_launches(recorded, n, offset, dtype, kernels):
+    """One kernel for at most 262144 16-bit elements in whole aligned vectors, else a maximum and a conversion pass."""
+    x = torch.randn(n + offset, device=DEV).to(dtype)[offset:]
+    before = _lib.launch_count
+    with _lib.record_kernel_times() if recorded else torch.enable_grad():
+        quantize_fp8(x, E4, G.TENSORWISE)
+    assert _lib.launch_count - before == kernels
+
+
+@pytest.mark.parametrize("recorded", [False, True])
+def test_rowwise_quantise_counts_the_kernels_it_launches(recorded):
+    x = _rand(64, 256)
+    for axis, kernels in ((1, 1), (0, 2)):
+        before = _lib.launch_count
+        with _lib.record_kernel_times() if recorded else torch.enable_grad():
+            quantize_fp8(x, E4, G.ROWWISE, axis=axis)
+        assert _lib.launch_count - before == kernels
 
 
 # ---- weights quantised ahead of time ----------------------------------------------------------------------------
