@@ -123,6 +123,7 @@ _GEMM_ENTRY_POINTS = ("ptb_gemm_fp8", "ptb_gemm_mxfp8", "ptb_grouped_gemm_fp8", 
 # PTB_NVTX=1: one NVTX range per C-ABI call, named after the entry point (timeline tools show them)
 _NVTX = os.environ.get("PTB_NVTX", "0") not in ("", "0")
 _event_log = None  # when a dict: name -> [(start_event, stop_event), ...] on the launching stream
+_set_native_recording = lambda on: None  # noqa: E731  (the native host path's switch, once that is loaded)
 
 
 def call(name: str, *args) -> None:
@@ -189,11 +190,13 @@ class record_kernel_times:
         global _event_log
         self._prev, _event_log = _event_log, {}
         self.log = _event_log
+        _set_native_recording(True)
         return self
 
     def __exit__(self, *exc):
         global _event_log
         _event_log = self._prev
+        _set_native_recording(_event_log is not None)
         return False
 
     def durations_ms(self):

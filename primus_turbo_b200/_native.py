@@ -3,7 +3,7 @@
 The extension does what the Python wrappers in ``pytorch/kernels`` and the autograd Functions in ``pytorch/ops`` do
 -- check, allocate, launch, save for backward -- without the interpreter in between.  Those remain for what needs
 Python: traced calls, dispatch modes, tensor subclasses other than a cached weight, and per-kernel timing or NVTX
-ranges.  An entry of the extension returns ``None`` for arguments it does not handle, and the caller goes on in Python.
+ranges (a backward pass whose forward pass ran before the recording began is timed natively).  An entry of the extension returns ``None`` for arguments it does not handle, and the caller goes on in Python.
 """
 
 from __future__ import annotations
@@ -25,11 +25,14 @@ def _load():
     loader = ExtensionFileLoader("ptb_torch", str(_PATH))
     module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("ptb_torch", _PATH, loader=loader))
     loader.exec_module(module)
-    module.setup(_lib.PtbError, _lib._DEBUG_STATUS)
+    module.setup(_lib.PtbError, _lib.timed_region)
+    module.set_check_status(_lib._DEBUG_STATUS)
     return module
 
 
 ext = _load()
+_lib._set_native_recording = ext.set_recording
+ext.set_recording(_lib._event_log is not None)
 _PLAIN = (torch.Tensor, torch.nn.Parameter)
 
 

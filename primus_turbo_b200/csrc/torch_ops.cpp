@@ -40,7 +40,8 @@ constexpr int64_t kBlk = 128, kMxBlk = 32;
 
 std::atomic<int64_t> g_calls{0}; // C-ABI calls that enqueued work from here
 std::atomic<bool> g_check_status{false}; // debug: wait for the device after every GEMM and read the status word
-PyObject *g_error_class = nullptr;
+std::atomic<bool> g_recording{false};    // per-kernel times are being recorded
+PyObject *g_error_class = nullptr, *g_timed_region = nullptr;
 
 struct PtbFail : std::runtime_error {
     using std::runtime_error::runtime_error;
@@ -48,11 +49,27 @@ struct PtbFail : std::runtime_error {
 
 void check(int rc, const char *what) {
     if (rc != 0) throw PtbFail(std::string(what) + " failed with status " + std::to_string(rc) + ": " + ptb_last_error());
+}
+
+// One C-ABI call.  While per-kernel times are recorded -- a backward pass may meet that although its forward pass did not --
+// the recorder's own context manager brackets it with events.
+template <typename F> void run(const char *what, F &&f) {
+    int rc;
+    if (g_recording.load(std::memory_order_relaxed)) {
+        py::gil_scoped_acquire gil;
+        py::object region = py::handle(g_timed_region)(what);
+        region.attr("__enter__")();
+        rc = f();
+        region.attr("__exit__")(py::none(), py::none(), py::none());
+    } else {
+        rc = f();
+    }
+    check(rc, what);
     g_calls.fetch_add(1, std::memory_order_relaxed);
 }
 
-void check_gemm(int rc, const char *what, cudaStream_t st) {
-    check(rc, what);
+template <typename F> void run_gemm(const char *what, cudaStream_t st, F &&f) {
+    run(what, f);
     if (!g_check_status.load(std::memory_order_relaxed)) return;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return;
@@ -63,6 +80,9 @@ void check_gemm(int rc, const char *what, cudaStream_t st) {
         throw PtbFail(std::string(what) + ": a device-side wait ran out (status " + std::to_string(code) +
                       "); the output is incomplete");
 }
+
+#define PTB_RUN(fn, ...) run(#fn, [&] { return fn(__VA_ARGS__); })
+#define PTB_RUN_GEMM(fn, ...) run_gemm(#fn, c.st, [&] { return fn(__VA_ARGS__); })
 
 int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 int64_t round_up(int64_t a, int64_t b) { return cdiv(a, b) * b; }
@@ -106,9 +126,8 @@ struct Quant {
 Quant quant_tensorwise(const Call &c, const Tensor &x, ScalarType dt) {
     Quant r{c.empty(x.sizes(), dt), c.empty({}, ScalarType::Float)};
     Tensor ws = c.empty({PTB_TENSORWISE_WS_BYTES}, ScalarType::Byte);
-    check(ptb_quant_fp8_tensorwise(x.const_data_ptr(), code_of(x.scalar_type()), x.numel(), r.q.mutable_data_ptr(), code_of(dt),
-                                   r.s.mutable_data_ptr<float>(), ws.mutable_data_ptr(), c.st),
-          "ptb_quant_fp8_tensorwise");
+    PTB_RUN(ptb_quant_fp8_tensorwise, x.const_data_ptr(), code_of(x.scalar_type()), x.numel(), r.q.mutable_data_ptr(),
+            code_of(dt), r.s.mutable_data_ptr<float>(), ws.mutable_data_ptr(), c.st);
     return r;
 }
 
@@ -124,9 +143,8 @@ Quant quant_rowwise(const Call &c, const Tensor &x, ScalarType dt, int64_t axis)
     r.sm = 1;
     Tensor ws;
     if (N > 1) ws = c.empty({B * N}, ScalarType::Float);
-    check(ptb_quant_fp8_rowwise(x.const_data_ptr(), code_of(x.scalar_type()), B, M, N, r.q.mutable_data_ptr(), code_of(dt),
-                                r.s.mutable_data_ptr<float>(), N > 1 ? ws.mutable_data_ptr() : nullptr, c.st),
-          "ptb_quant_fp8_rowwise");
+    PTB_RUN(ptb_quant_fp8_rowwise, x.const_data_ptr(), code_of(x.scalar_type()), B, M, N, r.q.mutable_data_ptr(), code_of(dt),
+            r.s.mutable_data_ptr<float>(), N > 1 ? ws.mutable_data_ptr() : nullptr, c.st);
     return r;
 }
 
@@ -136,9 +154,8 @@ Tensor dequant_rowwise(const Call &c, const Tensor &q, const Tensor &s, ScalarTy
     for (int64_t i = 0; i < axis; ++i) B *= q.size(i);
     for (int64_t i = axis + 1; i < q.dim(); ++i) N *= q.size(i);
     Tensor out = c.empty(q.sizes(), dt);
-    check(ptb_dequant_fp8_rowwise(q.const_data_ptr(), code_of(q.scalar_type()), B, q.size(axis), N, s.const_data_ptr<float>(),
-                                  out.mutable_data_ptr(), code_of(dt), c.st),
-          "ptb_dequant_fp8_rowwise");
+    PTB_RUN(ptb_dequant_fp8_rowwise, q.const_data_ptr(), code_of(q.scalar_type()), B, q.size(axis), N,
+            s.const_data_ptr<float>(), out.mutable_data_ptr(), code_of(dt), c.st);
     return out;
 }
 
@@ -154,27 +171,24 @@ Quant requant_rowwise(const Call &c, const Quant &r, ScalarType hp, int64_t have
     Quant o{c.empty(r.q.sizes(), r.q.scalar_type()), c.empty(sshape, ScalarType::Float)};
     o.sm      = 1;
     Tensor ws = c.empty({B * N}, ScalarType::Float);
-    check(ptb_requant_fp8_rowwise(r.q.const_data_ptr(), code_of(r.q.scalar_type()), r.scale(), code_of(hp), B, M, N,
-                                  o.q.mutable_data_ptr(), o.s.mutable_data_ptr<float>(), ws.mutable_data_ptr(), c.st),
-          "ptb_requant_fp8_rowwise");
+    PTB_RUN(ptb_requant_fp8_rowwise, r.q.const_data_ptr(), code_of(r.q.scalar_type()), r.scale(), code_of(hp), B, M, N,
+            o.q.mutable_data_ptr(), o.s.mutable_data_ptr<float>(), ws.mutable_data_ptr(), c.st);
     return o;
 }
 
 Quant quant_block_rows(const Call &c, const Tensor &x, ScalarType dt) {
     const int64_t M = x.size(0), N = x.size(1), nb = cdiv(N, kBlk);
     Quant r{c.empty({M, N}, dt), c.empty({M, nb}, ScalarType::Float), nb, 1};
-    check(ptb_quant_fp8_block1d(x.const_data_ptr(), code_of(x.scalar_type()), M, N, 1, r.q.mutable_data_ptr(), code_of(dt),
-                                r.s.mutable_data_ptr<float>(), c.st),
-          "ptb_quant_fp8_block1d");
+    PTB_RUN(ptb_quant_fp8_block1d, x.const_data_ptr(), code_of(x.scalar_type()), M, N, 1, r.q.mutable_data_ptr(), code_of(dt),
+            r.s.mutable_data_ptr<float>(), c.st);
     return r;
 }
 
 Quant quant_block_cols(const Call &c, const Tensor &x, ScalarType dt) {
     const int64_t M = x.size(0), N = x.size(1);
     Quant r{c.empty({M, N}, dt), c.empty({cdiv(M, kBlk), N}, ScalarType::Float), 1, N};
-    check(ptb_quant_fp8_block1d(x.const_data_ptr(), code_of(x.scalar_type()), M, N, 0, r.q.mutable_data_ptr(), code_of(dt),
-                                r.s.mutable_data_ptr<float>(), c.st),
-          "ptb_quant_fp8_block1d");
+    PTB_RUN(ptb_quant_fp8_block1d, x.const_data_ptr(), code_of(x.scalar_type()), M, N, 0, r.q.mutable_data_ptr(), code_of(dt),
+            r.s.mutable_data_ptr<float>(), c.st);
     return r;
 }
 
@@ -182,10 +196,8 @@ std::pair<Quant, Quant> quant_block_dual(const Call &c, const Tensor &x, ScalarT
     const int64_t M = x.size(0), N = x.size(1), nb = cdiv(N, kBlk);
     Quant row{c.empty({M, N}, dt), c.empty({M, nb}, ScalarType::Float), nb, 1};
     Quant col{c.empty({M, N}, dt), c.empty({cdiv(M, kBlk), N}, ScalarType::Float), 1, N};
-    check(ptb_quant_fp8_block1d_dual(x.const_data_ptr(), code_of(x.scalar_type()), M, N, row.q.mutable_data_ptr(),
-                                     row.s.mutable_data_ptr<float>(), col.q.mutable_data_ptr(), col.s.mutable_data_ptr<float>(),
-                                     code_of(dt), c.st),
-          "ptb_quant_fp8_block1d_dual");
+    PTB_RUN(ptb_quant_fp8_block1d_dual, x.const_data_ptr(), code_of(x.scalar_type()), M, N, row.q.mutable_data_ptr(),
+            row.s.mutable_data_ptr<float>(), col.q.mutable_data_ptr(), col.s.mutable_data_ptr<float>(), code_of(dt), c.st);
     return {row, col};
 }
 
@@ -195,9 +207,8 @@ Quant quant_block_tiles(const Call &c, const Tensor &w, ScalarType dt) {
     const int64_t B = batched ? w.size(0) : 1, M = w.size(-2), N = w.size(-1), mb = cdiv(M, kBlk), nb = cdiv(N, kBlk);
     Quant r{c.empty(w.sizes(), dt), batched ? c.empty({B, mb, nb}, ScalarType::Float) : c.empty({mb, nb}, ScalarType::Float),
             nb, 1, mb * nb};
-    check(ptb_quant_fp8_block2d(w.const_data_ptr(), code_of(w.scalar_type()), B, M, N, r.q.mutable_data_ptr(), code_of(dt),
-                                r.s.mutable_data_ptr<float>(), c.st),
-          "ptb_quant_fp8_block2d");
+    PTB_RUN(ptb_quant_fp8_block2d, w.const_data_ptr(), code_of(w.scalar_type()), B, M, N, r.q.mutable_data_ptr(), code_of(dt),
+            r.s.mutable_data_ptr<float>(), c.st);
     return r;
 }
 
@@ -213,10 +224,10 @@ std::pair<Quant, Quant> quant_mx(const Call &c, const Tensor &x, ScalarType dt, 
     Quant row, col;
     if (want_row) row = {make(M, Np, dt), make(M, Np / kMxBlk, ScalarType::Byte)};
     if (want_col) col = {make(N, Mp, dt), make(N, Mp / kMxBlk, ScalarType::Byte)};
-    check(ptb_quant_mxfp8(x.const_data_ptr(), code_of(x.scalar_type()), G, M, N, want_row ? row.q.mutable_data_ptr() : nullptr,
-                          want_row ? row.s.mutable_data_ptr() : nullptr, want_col ? col.q.mutable_data_ptr() : nullptr,
-                          want_col ? col.s.mutable_data_ptr() : nullptr, row_2d, col_2d, code_of(dt), c.st),
-          "ptb_quant_mxfp8");
+    PTB_RUN(ptb_quant_mxfp8, x.const_data_ptr(), code_of(x.scalar_type()), G, M, N,
+            want_row ? row.q.mutable_data_ptr() : nullptr, want_row ? row.s.mutable_data_ptr() : nullptr,
+            want_col ? col.q.mutable_data_ptr() : nullptr, want_col ? col.s.mutable_data_ptr() : nullptr, row_2d, col_2d,
+            code_of(dt), c.st);
     return {row, col};
 }
 
@@ -229,20 +240,18 @@ Tensor gemm(const Call &c, const Quant &a, bool ta, const Quant &b, bool tb, Sca
     Tensor out = c.empty({M, N}, out_dt);
     int64_t asm_ = a.sm, ask = a.sk, bsn = b.sm, bsk = b.sk;
     if (gran == PTB_BLOCKWISE && b_tiles && !tb) std::swap(bsn, bsk); // tile scales are stored like the matrix: [K/128, N/128]
-    check_gemm(ptb_gemm_fp8(a.q.const_data_ptr(), code_of(a.q.scalar_type()), ta, a.q.size(1), b.q.const_data_ptr(),
-                            code_of(b.q.scalar_type()), tb, b.q.size(1), out.mutable_data_ptr(), code_of(out_dt), N, M, N, K, gran,
-                            a.scale(), asm_, ask, b.scale(), bsn, bsk, b_tiles, 0, c.st),
-               "ptb_gemm_fp8", c.st);
+    PTB_RUN_GEMM(ptb_gemm_fp8, a.q.const_data_ptr(), code_of(a.q.scalar_type()), ta, a.q.size(1), b.q.const_data_ptr(),
+                 code_of(b.q.scalar_type()), tb, b.q.size(1), out.mutable_data_ptr(), code_of(out_dt), N, M, N, K, gran,
+                 a.scale(), asm_, ask, b.scale(), bsn, bsk, b_tiles, 0, c.st);
     return out;
 }
 
 Tensor gemm_mx(const Call &c, const Quant &a, const Quant &b, ScalarType out_dt) {
     const int64_t M = a.q.size(0), K = a.q.size(1), N = b.q.size(0);
     Tensor out = c.empty({M, N}, out_dt);
-    check_gemm(ptb_gemm_mxfp8(a.q.const_data_ptr(), code_of(a.q.scalar_type()), K, a.s.const_data_ptr(), a.s.size(1),
-                              b.q.const_data_ptr(), code_of(b.q.scalar_type()), K, b.s.const_data_ptr(), b.s.size(1),
-                              out.mutable_data_ptr(), code_of(out_dt), N, M, N, K, 0, c.st),
-               "ptb_gemm_mxfp8", c.st);
+    PTB_RUN_GEMM(ptb_gemm_mxfp8, a.q.const_data_ptr(), code_of(a.q.scalar_type()), K, a.s.const_data_ptr(), a.s.size(1),
+                 b.q.const_data_ptr(), code_of(b.q.scalar_type()), K, b.s.const_data_ptr(), b.s.size(1), out.mutable_data_ptr(),
+                 code_of(out_dt), N, M, N, K, 0, c.st);
     return out;
 }
 
@@ -349,7 +358,7 @@ struct Layout {
 
 Tensor group_offsets(const Call &c, const Tensor &lens) {
     Tensor offs = c.empty({lens.numel() + 1}, ScalarType::Long);
-    check(ptb_group_offs(lens.const_data_ptr<int64_t>(), lens.numel(), offs.mutable_data_ptr<int64_t>(), c.st), "ptb_group_offs");
+    PTB_RUN(ptb_group_offs, lens.const_data_ptr<int64_t>(), lens.numel(), offs.mutable_data_ptr<int64_t>(), c.st);
     return offs;
 }
 
@@ -361,11 +370,10 @@ std::pair<Quant, Quant> quant_segments(const Call &c, const Tensor &x, ScalarTyp
     Tensor pads = c.empty({2 * G + 1}, ScalarType::Long);
     Tensor table = c.empty({cdiv(Mp, kBlk), 2}, ScalarType::Int);
     int64_t *p = pads.mutable_data_ptr<int64_t>();
-    check(ptb_quant_fp8_segment_row_col(x.const_data_ptr(), code_of(x.scalar_type()), M, N, G, lens.const_data_ptr<int64_t>(),
-                                        l.offs.const_data_ptr<int64_t>(), row.q.mutable_data_ptr(), col.q.mutable_data_ptr(),
-                                        row.s.mutable_data_ptr<float>(), col.s.mutable_data_ptr<float>(), p + G + 1, p,
-                                        table.mutable_data_ptr(), code_of(dt), c.st),
-          "ptb_quant_fp8_segment_row_col");
+    PTB_RUN(ptb_quant_fp8_segment_row_col, x.const_data_ptr(), code_of(x.scalar_type()), M, N, G,
+            lens.const_data_ptr<int64_t>(), l.offs.const_data_ptr<int64_t>(), row.q.mutable_data_ptr(),
+            col.q.mutable_data_ptr(), row.s.mutable_data_ptr<float>(), col.s.mutable_data_ptr<float>(), p + G + 1, p,
+            table.mutable_data_ptr(), code_of(dt), c.st);
     l.padded = pads; // first G + 1 words: the padded offsets
     return {row, col};
 }
@@ -377,11 +385,9 @@ std::pair<Quant, Quant> quant_mx_groups(const Call &c, const Tensor &x, ScalarTy
     Tensor pads = c.empty({4 * G + 2}, ScalarType::Long);
     Tensor table = c.empty({Mc / kBlk * 4}, ScalarType::Int);
     int64_t *p = pads.mutable_data_ptr<int64_t>(); // column offsets first: they are what wgrad reads
-    check(ptb_quant_mxfp8_grouped(x.const_data_ptr(), code_of(x.scalar_type()), M, N, l.offs.const_data_ptr<int64_t>(), G, 1,
-                                  row.q.mutable_data_ptr(), row.s.mutable_data_ptr(), col.q.mutable_data_ptr(),
-                                  col.s.mutable_data_ptr(), p + G + 1, p + 2 * G + 1, p + 3 * G + 2, p, table.mutable_data_ptr(),
-                                  0, 0, code_of(dt), c.st),
-          "ptb_quant_mxfp8_grouped");
+    PTB_RUN(ptb_quant_mxfp8_grouped, x.const_data_ptr(), code_of(x.scalar_type()), M, N, l.offs.const_data_ptr<int64_t>(), G, 1,
+            row.q.mutable_data_ptr(), row.s.mutable_data_ptr(), col.q.mutable_data_ptr(), col.s.mutable_data_ptr(), p + G + 1,
+            p + 2 * G + 1, p + 3 * G + 2, p, table.mutable_data_ptr(), 0, 0, code_of(dt), c.st);
     l.padded = pads;
     return {row, col};
 }
@@ -392,11 +398,9 @@ Tensor grouped_gemm(const Call &c, const Quant &a, const Quant &b, bool tb, cons
     int64_t bsg = b.sg, bsn = b.sm, bsk = b.sk;
     if (d.gran == PTB_BLOCKWISE && !tb) std::swap(bsn, bsk);
     if (d.gran == PTB_ROWWISE) bsg = N;
-    check_gemm(ptb_grouped_gemm_fp8(a.q.const_data_ptr(), code_of(a.q.scalar_type()), K, b.q.const_data_ptr(),
-                                    code_of(b.q.scalar_type()), tb, out.mutable_data_ptr(), code_of(d.out), N,
-                                    offs.const_data_ptr<int64_t>(), G, M, N, K, d.gran, a.scale(), a.sm, a.sk, b.scale(), bsg, bsn,
-                                    bsk, d.num_sms, c.st),
-               "ptb_grouped_gemm_fp8", c.st);
+    PTB_RUN_GEMM(ptb_grouped_gemm_fp8, a.q.const_data_ptr(), code_of(a.q.scalar_type()), K, b.q.const_data_ptr(),
+                 code_of(b.q.scalar_type()), tb, out.mutable_data_ptr(), code_of(d.out), N, offs.const_data_ptr<int64_t>(), G,
+                 M, N, K, d.gran, a.scale(), a.sm, a.sk, b.scale(), bsg, bsn, bsk, d.num_sms, c.st);
     return out;
 }
 
@@ -404,32 +408,28 @@ Tensor grouped_gemm(const Call &c, const Quant &a, const Quant &b, bool tb, cons
 Tensor grouped_wgrad(const Call &c, const Quant &lhs, const Quant &rhs, const Tensor &offs, int64_t G, const GroupedSpec &d) {
     const int64_t rows = lhs.q.size(0), OM = lhs.q.size(1), ON = rhs.q.size(1);
     Tensor out = c.empty({G, OM, ON}, d.out);
-    check_gemm(ptb_grouped_gemm_fp8_variable_k(lhs.q.const_data_ptr(), code_of(lhs.q.scalar_type()), OM, rhs.q.const_data_ptr(),
-                                               code_of(rhs.q.scalar_type()), ON, out.mutable_data_ptr(), code_of(d.out),
-                                               offs.const_data_ptr<int64_t>(), G, rows, OM, ON, d.gran, lhs.scale(), rhs.scale(),
-                                               d.num_sms, c.st),
-               "ptb_grouped_gemm_fp8_variable_k", c.st);
+    PTB_RUN_GEMM(ptb_grouped_gemm_fp8_variable_k, lhs.q.const_data_ptr(), code_of(lhs.q.scalar_type()), OM,
+                 rhs.q.const_data_ptr(), code_of(rhs.q.scalar_type()), ON, out.mutable_data_ptr(), code_of(d.out),
+                 offs.const_data_ptr<int64_t>(), G, rows, OM, ON, d.gran, lhs.scale(), rhs.scale(), d.num_sms, c.st);
     return out;
 }
 
 Tensor grouped_gemm_mx(const Call &c, const Quant &a, const Quant &b, const Tensor &offs, const GroupedSpec &d) {
     const int64_t M = a.q.size(0), K = a.q.size(1), G = b.q.size(0), N = b.q.size(1);
     Tensor out = c.empty({M, N}, d.out);
-    check_gemm(ptb_grouped_gemm_mxfp8(a.q.const_data_ptr(), code_of(a.q.scalar_type()), K, a.s.const_data_ptr(), a.s.size(1),
-                                      b.q.const_data_ptr(), code_of(b.q.scalar_type()), b.s.const_data_ptr(), out.mutable_data_ptr(),
-                                      code_of(d.out), N, offs.const_data_ptr<int64_t>(), G, M, N, K, d.num_sms, c.st),
-               "ptb_grouped_gemm_mxfp8", c.st);
+    PTB_RUN_GEMM(ptb_grouped_gemm_mxfp8, a.q.const_data_ptr(), code_of(a.q.scalar_type()), K, a.s.const_data_ptr(), a.s.size(1),
+                 b.q.const_data_ptr(), code_of(b.q.scalar_type()), b.s.const_data_ptr(), out.mutable_data_ptr(), code_of(d.out),
+                 N, offs.const_data_ptr<int64_t>(), G, M, N, K, d.num_sms, c.st);
     return out;
 }
 
 Tensor grouped_wgrad_mx(const Call &c, const Quant &lhs, const Quant &rhs, const Tensor &offs, int64_t G, const GroupedSpec &d) {
     const int64_t OM = lhs.q.size(0), ON = rhs.q.size(0), rows = lhs.q.size(1);
     Tensor out = c.empty({G, OM, ON}, d.out);
-    check_gemm(ptb_grouped_gemm_mxfp8_variable_k(lhs.q.const_data_ptr(), code_of(lhs.q.scalar_type()), rows, lhs.s.const_data_ptr(),
-                                                 lhs.s.size(1), rhs.q.const_data_ptr(), code_of(rhs.q.scalar_type()), rows,
-                                                 rhs.s.const_data_ptr(), rhs.s.size(1), out.mutable_data_ptr(), code_of(d.out),
-                                                 offs.const_data_ptr<int64_t>(), G, rows, OM, ON, d.num_sms, c.st),
-               "ptb_grouped_gemm_mxfp8_variable_k", c.st);
+    PTB_RUN_GEMM(ptb_grouped_gemm_mxfp8_variable_k, lhs.q.const_data_ptr(), code_of(lhs.q.scalar_type()), rows,
+                 lhs.s.const_data_ptr(), lhs.s.size(1), rhs.q.const_data_ptr(), code_of(rhs.q.scalar_type()), rows,
+                 rhs.s.const_data_ptr(), rhs.s.size(1), out.mutable_data_ptr(), code_of(d.out), offs.const_data_ptr<int64_t>(),
+                 G, rows, OM, ON, d.num_sms, c.st);
     return out;
 }
 
@@ -757,22 +757,18 @@ py::object py_dequantize(const Tensor &q, const Tensor &s, ScalarType out_dt, in
         void *o = out.mutable_data_ptr();
         switch (gran) {
         case PTB_TENSORWISE:
-            check(ptb_dequant_fp8_tensorwise(q.const_data_ptr(), qc, q.numel(), s.const_data_ptr<float>(), o, oc, c.st),
-                  "ptb_dequant_fp8_tensorwise");
+            PTB_RUN(ptb_dequant_fp8_tensorwise, q.const_data_ptr(), qc, q.numel(), s.const_data_ptr<float>(), o, oc, c.st);
             break;
         case PTB_BLOCKWISE:
             if (tiles)
-                check(ptb_dequant_fp8_block2d(q.const_data_ptr(), qc, nd == 3 ? q.size(0) : 1, q.size(-2), q.size(-1),
-                                              s.const_data_ptr<float>(), o, oc, c.st),
-                      "ptb_dequant_fp8_block2d");
+                PTB_RUN(ptb_dequant_fp8_block2d, q.const_data_ptr(), qc, nd == 3 ? q.size(0) : 1, q.size(-2), q.size(-1),
+                        s.const_data_ptr<float>(), o, oc, c.st);
             else
-                check(ptb_dequant_fp8_block1d(q.const_data_ptr(), qc, q.size(0), q.size(1), axis == 1,
-                                              s.const_data_ptr<float>(), o, oc, c.st),
-                      "ptb_dequant_fp8_block1d");
+                PTB_RUN(ptb_dequant_fp8_block1d, q.const_data_ptr(), qc, q.size(0), q.size(1), axis == 1,
+                        s.const_data_ptr<float>(), o, oc, c.st);
             break;
         default:
-            check(ptb_dequant_mxfp8(q.const_data_ptr(), qc, q.size(0), q.size(1), s.const_data_ptr(), flip, o, oc, c.st),
-                  "ptb_dequant_mxfp8");
+            PTB_RUN(ptb_dequant_mxfp8, q.const_data_ptr(), qc, q.size(0), q.size(1), s.const_data_ptr(), flip, o, oc, c.st);
         }
         return py::cast(out);
     });
@@ -782,10 +778,12 @@ py::object py_dequantize(const Tensor &q, const Tensor &s, ScalarType out_dt, in
 
 PYBIND11_MODULE(ptb_torch, m) {
     m.doc() = "native host path of the FP8 ops";
-    m.def("setup", [](py::object error_class, bool check_status) {
-        g_error_class = error_class.release().ptr(); // kept for the life of the process
-        g_check_status = check_status;
+    m.def("setup", [](py::object error_class, py::object timed_region) {
+        g_error_class  = error_class.release().ptr(); // both kept for the life of the process
+        g_timed_region = timed_region.release().ptr();
     });
+    m.def("set_check_status", [](bool on) { g_check_status = on; });
+    m.def("set_recording", [](bool on) { g_recording = on; });
     m.def("calls", [] { return g_calls.load(std::memory_order_relaxed); });
     m.def("gemm_fp8", &py_gemm_fp8);
     m.def("grouped_gemm_fp8", &py_grouped_gemm_fp8);

@@ -73,6 +73,31 @@ def test_a_traced_call_runs_again_on_new_inputs(gran, grouped):
     assert torch.equal(traced(a), op(a, w))
 
 
+# ---- per-kernel times -------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("grouped", [False, True])
+@pytest.mark.parametrize("gran", GRANS)
+def test_kernel_times_of_a_backward_whose_forward_ran_before(gran, grouped):
+    op, a, w = _op(grouped, gran)
+    a.requires_grad_(), w.requires_grad_()
+
+    def log_of(forward_inside):
+        with _lib.record_kernel_times() if forward_inside else torch.enable_grad():
+            out = op(a, w)
+        with _lib.record_kernel_times() as rec:
+            torch.autograd.grad(out, (a, w), torch.ones_like(out))
+        times = rec.durations_ms()
+        assert all(t >= 0 for v in times.values() for t in v)
+        # (the Python form of a grouped backward pass derives the group offsets once more)
+        return {name: len(v) for name, v in times.items() if name != "ptb_group_offs"}
+
+    native, python = log_of(False), log_of(True)
+    assert native == python and any("gemm" in name for name in native)
+    with _lib.record_kernel_times() as rec:
+        pass
+    out = op(a, w)  # and nothing is logged once recording has ended
+    assert rec.log == {}
+
+
 # ---- kernel counts ----------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("recorded", [False, True])
 @pytest.mark.parametrize("n,offset,dtype,kernels", [
