@@ -46,3 +46,41 @@ def test_groups_equal_the_general_kernel(gran, lens, tail):
     want = grouped_gemm_fp8(more, w, torch.tensor(lens, device="cuda"), config=_config(gran))
     assert torch.equal(out[: sum(lens)], want[: sum(lens)])
     assert not out[sum(lens) :].any() and not want[sum(lens) :].any()
+
+
+def _grads(op, x, w, gy):
+    x, w = x.detach().requires_grad_(), w.detach().requires_grad_()
+    return torch.autograd.grad(op(x, w), (x, w), gy)
+
+
+@pytest.mark.parametrize("gran", GRANS)
+@pytest.mark.parametrize("n,k", [(128, 256), (1040, 1200)])
+def test_dense_backward_of_few_rows_with_mixed_formats(gran, n, k):
+    """The gradient against a [K, N] weight is a product with a K-major weight: e5m2 rows, e4m3 weight."""
+    cfg = _config(gran)
+    cfg.format = Format.HYBRID
+    torch.manual_seed(n)
+    x, gy = torch.randn(300, k, device="cuda", dtype=torch.bfloat16), torch.randn(300, n, device="cuda", dtype=torch.bfloat16)
+    x[0, 0], gy[0, 0] = 16.0, 16.0  # the tensorwise scales are the same for every number of rows
+    w = torch.randn(k, n, device="cuda", dtype=torch.bfloat16)
+    op = lambda a, b: gemm_fp8(a, b, config=cfg)  # noqa: E731
+    full = _grads(op, x, w, gy)[0]
+    for m in (1, 31, 33, 64, 65, 128, 129):
+        assert torch.equal(_grads(op, x[:m], w, gy[:m])[0], full[:m]), m
+
+
+@pytest.mark.parametrize("gran", GRANS)
+@pytest.mark.parametrize("lens", [[8] * 12, [0, 65, 1, 0, 40, 0], [0, 0, 96, 0], [32, 33, 31, 0, 0], [0, 0, 0, 130, 0, 3, 0, 0]])
+def test_group_backward_of_few_rows_with_mixed_formats(gran, lens):
+    cfg = _config(gran)
+    cfg.format = Format.HYBRID
+    torch.manual_seed(len(lens))
+    g, n, k = len(lens), 528, 1168
+    rows, more = sum(lens), 33 * len(lens) + sum(lens)
+    x, gy = torch.randn(rows, k, device="cuda", dtype=torch.bfloat16), torch.randn(rows, n, device="cuda", dtype=torch.bfloat16)
+    w = torch.randn(g, k, n, device="cuda", dtype=torch.bfloat16)
+    op = lambda a, b: grouped_gemm_fp8(a, b, torch.tensor(lens, device="cuda"), trans_b=False, config=cfg)  # noqa: E731
+    got = _grads(op, x, w, gy)[0]
+    pad = lambda t: torch.cat([t, t.new_zeros(more - rows, t.shape[1])])  # noqa: E731
+    want = _grads(op, pad(x), w, pad(gy))[0]
+    assert torch.equal(got, want[:rows])
