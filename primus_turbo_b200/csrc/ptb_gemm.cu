@@ -1345,7 +1345,7 @@ int ptb_gemm_fp8(const void *a, int a_dtype, int trans_a, int64_t lda, const voi
     g.c = c; g.ldc = ldc; g.c_group_stride = 0;
     g.a_scale = a_scale; g.as_m = a_scale_stride_m; g.as_k = a_scale_stride_k;
     g.b_scale = b_scale; g.bs_g = 0; g.bs_n = b_scale_stride_n; g.bs_k = b_scale_stride_k;
-    if (const int tn = skinny_rows(mode, M, 0, !trans_a && trans_b))
+    if (const int tn = skinny_rows(mode, M, 0, N, !trans_a && trans_b, grid))
         return launch_skinny(g, mode, tn, a, a_dtype, lda, b, b_dtype, ldb, 1, c_dtype, grid, (cudaStream_t) stream);
     const int ctas = dense_ctas(mode, M, N, grid);
     set_tile(g, ctas);
@@ -1505,7 +1505,7 @@ int ptb_grouped_gemm_fp8(const void *a, int a_dtype, int64_t lda, const void *b,
     g.c = out; g.ldc = ldc; g.c_group_stride = 0;
     g.a_scale = a_scale; g.as_m = a_scale_stride_m; g.as_k = a_scale_stride_k;
     g.b_scale = b_scale; g.bs_g = b_scale_stride_g; g.bs_n = b_scale_stride_n; g.bs_k = b_scale_stride_k;
-    if (const int tn = skinny_rows(mode, M_total, G, trans_b != 0))
+    if (const int tn = skinny_rows(mode, M_total, G, N, trans_b != 0, grid))
         return launch_skinny(g, mode, tn, a, a_dtype, lda, b, b_dtype, K, (uint64_t) G, out_dtype, grid, (cudaStream_t) stream);
     const int ctas = grouped_ctas(mode, M_total, G, grid);
     set_tile(g, ctas);

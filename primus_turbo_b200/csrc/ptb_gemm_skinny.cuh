@@ -7,7 +7,7 @@
 // operands change places: 128 weight rows are the MMA's M side, TN = 32, 64 or 128 rows of `a` its N side, so twice the
 // tiles, a stage of 16 KiB of weight plus TN x 128 bytes, and an accumulator of TN columns.  A product's terms and
 // the order they are added in are the same, so the results are too.
-// 32 x 14336 x 4096 tensorwise: 19 -> 15 us; 32 experts x 4096 x 7168 blockwise, 256 rows: the whole call 201 -> 188 us.
+// 32 x 14336 x 4096 tensorwise: 19 -> 15 us; 32 experts x 4096 x 7168 tensorwise, 256 rows: the whole call 186 -> 175 us.
 //
 // One persistent CTA per SM, 256 threads: warp 0 TMA producer, warp 1 MMA issuer, warp 2 owns tensor memory, warp 3 loads
 // block scales, warps 4-7 read the accumulator (lane = weight row, registers = rows of `a`), scale and store: the 32
@@ -290,13 +290,18 @@ template <int SCALE> int launch_skinny_scale(const GemmArgs &args, int out_dtype
 }
 
 // Rows of `a` per tile for the swapped form, 0 where the 128 x 256 tile stays the better one.  Dense: all rows in one tile, so
-// that the weight is read once; from 129 rows on the ordinary tile's 128-row side is full.  Row groups: how the
-// rows are spread is known on the device only; the tile is twice the average group, and from 32 rows on average the
-// groups above it, each of which reads its expert's weight once per tile, cost what the others gain.
-int skinny_rows(int mode, int64_t rows, int64_t G, bool k_major) {
+// that the weight is read once; from 129 rows on the ordinary tile's 128-row side is full.
+// Row groups: how the rows are spread is known on the device only, and a group of more than 32 rows reads its expert's
+// weight once per 32.  So the line lies where a skewed load costs little: 32 experts x 4096 x 7168, tensorwise, ordinary
+// against swapped, softmax loads of 8 rows a group 186 against 175 us, of 16 193 against 197; the same rows on two experts
+// 53 against 59 and 57 against 98.  With block scales every further tile promotes its own partial products, and only
+// calls that cannot give every SM an ordinary tile stay here (64 rows on two experts 46 against 38 us; softmax loads of 4,
+// 12 and 24 rows a group 149, 187, 189 against 163, 210, 237).
+int skinny_rows(int mode, int64_t rows, int64_t G, int64_t N, bool k_major, int grid) {
     if (!k_major || (mode != kScaleTensor && mode != kScaleRow && mode != kScaleBlock2D)) return 0;
     if (G == 0) return rows <= 32 ? 32 : rows <= 64 ? 64 : rows <= 128 ? 128 : 0;
-    return rows <= 16 * G ? 32 : rows <= 32 * G ? 64 : 0;
+    const bool few_tiles = rows * cdiv<int64_t>(N, kTileN) <= grid; // even if every row has an expert of its own
+    return few_tiles || (mode != kScaleBlock2D && rows <= 8 * G) ? 32 : 0;
 }
 
 // `a` [M, K] and `w` [G or 1, N, K] (both K-major), as the entry points got them

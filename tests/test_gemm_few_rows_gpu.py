@@ -31,7 +31,8 @@ def test_dense_rows_equal_the_general_kernel(gran, n, k, dtype):
 
 
 @pytest.mark.parametrize("gran", GRANS)
-@pytest.mark.parametrize("lens", [[8] * 12, [0, 65, 1, 0, 40, 0], [0, 0, 96, 0], [32, 33, 31, 0, 0]])
+@pytest.mark.parametrize("lens", [[8] * 12, [0, 65, 1, 0, 40, 0], [0, 0, 96, 0], [32, 33, 31, 0, 0],
+                                  [0] * 9 + [33, 0, 1, 65, 32] + [0] * 6, [5, 0, 33, 1, 0, 0]])
 @pytest.mark.parametrize("tail", [0, 7])
 def test_groups_equal_the_general_kernel(gran, lens, tail):
     torch.manual_seed(len(lens))
@@ -70,7 +71,8 @@ def test_dense_backward_of_few_rows_with_mixed_formats(gran, n, k):
 
 
 @pytest.mark.parametrize("gran", GRANS)
-@pytest.mark.parametrize("lens", [[8] * 12, [0, 65, 1, 0, 40, 0], [0, 0, 96, 0], [32, 33, 31, 0, 0], [0, 0, 0, 130, 0, 3, 0, 0]])
+@pytest.mark.parametrize("lens", [[8] * 12, [0, 65, 1, 0, 40, 0], [0, 0, 96, 0], [32, 33, 31, 0, 0], [0, 0, 0, 130, 0, 3, 0, 0],
+                                  [0] * 9 + [33, 0, 1, 65, 32] + [0] * 6, [5, 0, 6, 1, 0, 0]])
 def test_group_backward_of_few_rows_with_mixed_formats(gran, lens):
     cfg = _config(gran)
     cfg.format = Format.HYBRID
